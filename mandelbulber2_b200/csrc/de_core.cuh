@@ -1610,6 +1610,95 @@ __device__ __forceinline__ int compute_orbit(const DevScene &sc, T px, T py, T p
   return i;
 }
 
+// The same orbit one pass of the loop at a time, for kernels whose lanes are
+// at different iterations of different points: 3-D, without the extended
+// features (F 0, 2, 7 or 8) and with every slot's weight 1.  Every operation and its order are those of
+// compute_orbit<T, F, false>, except that the bailout compares |z|^2 with the
+// largest square whose root passes (bailout.h: the same outcome for every
+// input), so only the Mandelbulb, whose formula reads r, takes a root per pass.
+//
+// In the kernels built with contraction (MBR_NO_FMA: without) the fused
+// operations are spelled out where a compiler's choice would depend on what
+// surrounds them, as compute_orbit's sequence iteration has them: the
+// c-addition takes the formula's result as addend, and |z|^2 of the starting
+// point fuses x before y, that of the later points y before x.
+template <class T>
+__device__ __forceinline__ T fused(T a, T b, T c) {
+#ifdef MBR_NO_FMA
+  return a * b + c;
+#else
+  if constexpr (sizeof(T) == 8) return __fma_rn(a, b, c);
+  else return __fmaf_rn(a, b, c);
+#endif
+}
+template <class T>
+__device__ __forceinline__ T add_julia(const DevScene &sc, T z, int k) {
+  if constexpr (sizeof(T) == 8) return fused<T>(sc.julia_c[k], sc.cmul[k], z);
+  else return __fadd_rn(z, juliac_of<T>(sc, k));
+}
+template <class T>
+__device__ __forceinline__ T start_length(const V4<T> &z) {
+#ifdef MBR_NO_FMA
+  return len4<T, false>(z);
+#else
+  return m_sqrt(fused<T>(z.z, z.z, fused<T>(z.x, z.x, z.y * z.y)));
+#endif
+}
+enum OrbitEnd { ORBIT_RUNS = 0, ORBIT_MAXITER, ORBIT_NAN, ORBIT_BAILOUT };
+template <class T>
+struct OrbitLane {
+  T zx, zy, zz, cx, cy, cz, de;
+  int it;   // passes done
+  int end;  // OrbitEnd
+};
+template <class T>
+__device__ __forceinline__ void orbit_begin(OrbitLane<T> &e, T px, T py, T pz, int maxN) {
+  e.zx = e.cx = px;
+  e.zy = e.cy = py;
+  e.zz = e.cz = pz;
+  e.de = T(1.0);
+  e.it = 0;
+  e.end = maxN > 0 ? ORBIT_RUNS : ORBIT_MAXITER;
+}
+template <class T, int F>
+__device__ __forceinline__ void orbit_pass(const DevScene &sc, OrbitLane<T> &e, int maxN) {
+  const int i = e.it;
+  const int k = (F > 0) ? 0 : ((i < sc.length) ? int(sc.seq[i]) : int(sc.seq[0]));
+  const DevSlot &s = sc.slot[k];
+  V4<T> z{e.zx, e.zy, e.zz, T(0.0)};
+  const V4<T> last = z;
+  T de = e.de;
+  const int formula = F > 0 ? F : s.formula;
+  if (formula == MBR_FORMULA_MANDELBULB)
+    f_mandelbulb<T>(z, i == 0 ? start_length<T>(z) : len4<T, false>(z), de, s);
+  else if (formula == MBR_FORMULA_MANDELBOX)
+    f_mandelbox<T, false>(z, de, s);
+  else
+    f_menger<T, false>(z, de, s);
+  if (s.add_c) {
+    if (sc.julia) {
+      z.x = add_julia<T>(sc, z.x, 0);
+      z.y = add_julia<T>(sc, z.y, 1);
+      z.z = add_julia<T>(sc, z.z, 2);
+    } else {
+      z.x = fused<T>(e.cx, cmul_of<T>(sc, 0), z.x);
+      z.y = fused<T>(e.cy, cmul_of<T>(sc, 1), z.y);
+      z.z = fused<T>(e.cz, cmul_of<T>(sc, 2), z.z);
+    }
+  }
+  e.it = i + 1;
+  e.de = de;
+  if (nan4<T, false>(z)) {  // revert to the last finite orbit point
+    e.end = ORBIT_NAN;
+    return;
+  }
+  e.zx = z.x;
+  e.zy = z.y;
+  e.zz = z.z;
+  if (s.check_bailout && z.x * z.x + z.y * z.y + z.z * z.z > P<T>(s, P_BAILOUT_R2)) e.end = ORBIT_BAILOUT;
+  else if (e.it >= maxN) e.end = ORBIT_MAXITER;
+}
+
 // The final distance of an analytic orbit (compute_fractal.cpp:495-621).
 // The specialised iterations carry linear, logarithmic and IFS; the extended
 // one every DevDeFinal code.
@@ -1743,28 +1832,10 @@ __device__ __noinline__ T delta_distance(const DevScene &sc, T px, T py, T pz, T
   return distance;
 }
 
-// CalculateDistanceSimple (calculate_distance.cpp:533-760): the delta
-// branch (FP64) or the analytic branch, with its post-processing.  TREE: for
-// the fractal node nd of an explicit tree (its slot, iteration limit, julia
-// and constant factor, DE function).
-template <class T, int F, bool W, bool TREE = false>
-__device__ __forceinline__ T calc_distance_simple(const DevScene &sc, T px, T py, T pz, T detail, bool normal_mode,
-                                                  int *iters_out, int *total_out, const DevNode *nd = nullptr) {
-  if constexpr (F == F_EXT && sizeof(T) == 8) {
-    if (TREE ? nd->delta_de : sc.delta_de)
-      return delta_distance<T, W, TREE>(sc, px, py, pz, detail, normal_mode, iters_out, total_out, nd);
-  }
-  const int mult = (normal_mode && sc.iter_thresh) ? 5 : 1;
-  V4<T> z;
-  T r, DE, pk, cdist;
-  bool maxiter;
-  const int i = compute_orbit<T, F, W, TREE>(sc, px, py, pz, (TREE ? nd->maxN : sc.formula_maxiter) * mult, z, r,
-                                             DE, maxiter, nd, &pk, &cdist);
-  T distance = final_distance<T, F, W>(sc, z, r, DE, TREE ? nd->de_final : -1, pk, cdist);
-  const int iters = i + 1;
-  *iters_out = iters;
-  if (total_out) *total_out = iters;
-  // CalculateDistanceSimple post-processing (calculate_distance.cpp:561-605)
+// CalculateDistanceSimple post-processing (calculate_distance.cpp:561-605)
+template <class T>
+__device__ __forceinline__ T distance_tail(const DevScene &sc, T distance, int iters, bool maxiter, T detail,
+                                           bool normal_mode) {
   bool mx = maxiter;
   if (!sc.iter_thresh) mx = false;
   if (normal_mode) mx = false;
@@ -1783,6 +1854,30 @@ __device__ __forceinline__ T calc_distance_simple(const DevScene &sc, T px, T py
   if (distance < T(0.0)) distance = T(0.0);
   if (distance > T(10.0)) distance = T(10.0);
   return distance;
+}
+
+// CalculateDistanceSimple (calculate_distance.cpp:533-760): the delta
+// branch (FP64) or the analytic branch, with its post-processing.  TREE: for
+// the fractal node nd of an explicit tree (its slot, iteration limit, julia
+// and constant factor, DE function).
+template <class T, int F, bool W, bool TREE = false>
+__device__ __forceinline__ T calc_distance_simple(const DevScene &sc, T px, T py, T pz, T detail, bool normal_mode,
+                                                  int *iters_out, int *total_out, const DevNode *nd = nullptr) {
+  if constexpr (F == F_EXT && sizeof(T) == 8) {
+    if (TREE ? nd->delta_de : sc.delta_de)
+      return delta_distance<T, W, TREE>(sc, px, py, pz, detail, normal_mode, iters_out, total_out, nd);
+  }
+  const int mult = (normal_mode && sc.iter_thresh) ? 5 : 1;
+  V4<T> z;
+  T r, DE, pk, cdist;
+  bool maxiter;
+  const int i = compute_orbit<T, F, W, TREE>(sc, px, py, pz, (TREE ? nd->maxN : sc.formula_maxiter) * mult, z, r,
+                                             DE, maxiter, nd, &pk, &cdist);
+  const T distance = final_distance<T, F, W>(sc, z, r, DE, TREE ? nd->de_final : -1, pk, cdist);
+  const int iters = i + 1;
+  *iters_out = iters;
+  if (total_out) *total_out = iters;
+  return distance_tail<T>(sc, distance, iters, maxiter, detail, normal_mode);
 }
 
 // mergeChildIntoParent (calculate_distance.cpp:103-204) on the distance and

@@ -32,6 +32,7 @@ enum SlotParam {
   P_MB_OFF_Z,
   P_SCALE3,
   P_BAILOUT,
+  P_BAILOUT_R2,     // the largest r^2 whose square root rounds to at most the bailout (see orbit_pass)
   P_WEIGHT,
   P_AEX_CADD,       // aexion cadd
   P_ADE_ON,         // analyticDE enabled (0 or 1)

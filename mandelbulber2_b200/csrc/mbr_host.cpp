@@ -21,6 +21,7 @@
 
 #include "../../include/mbr.h"
 #include "mbr_device.h"
+#include "bailout.h"
 #include "mbr_internal.h"
 
 using namespace mbr;
@@ -591,8 +592,11 @@ mbr_status build_scene(mbr_ctx *ctx, const mbr_scene &sc, DevScene *out) {
   if (!any) return set_err(ctx, MBR_EINVAL, "scene has no formula");
   if (hybrid && sc.use_default_bailout)
     for (int i = 0; i < n; i++) d.slot[i].d[P_BAILOUT] = maxBailout;
-  for (int i = 0; i < MBR_MAX_FRACTALS; i++)
+  for (int i = 0; i < MBR_MAX_FRACTALS; i++) {
     for (int k = 0; k < P_COUNT; k++) d.slot[i].f[k] = float(d.slot[i].d[k]);
+    d.slot[i].d[P_BAILOUT_R2] = largest_square(d.slot[i].d[P_BAILOUT]);
+    d.slot[i].f[P_BAILOUT_R2] = largest_square(d.slot[i].f[P_BAILOUT]);
+  }
 
   // the sequence (hybrid_fractal_sequences.cpp:296-370)
   int length = MBR_SEQUENCE_LENGTH;

@@ -1,6 +1,7 @@
 // plain_fp64_strict.cu - the plain FP64 kernel compiled with --fmad=false:
 // every double operation is a separately rounded IEEE operation, in the
 // order the reference's CPU code performs them.
+#define MBR_NO_FMA 1
 #include "plain_kernel.cuh"
 
 namespace mbr {

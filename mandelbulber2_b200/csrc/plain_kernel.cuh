@@ -7,6 +7,8 @@
 // strict-FP64 (no FMA contraction) and mixed-precision builds of the same
 // template are distinct kernels.
 #pragma once
+#include <algorithm>
+
 #include "pixel_ops.cuh"
 
 namespace mbr {
@@ -208,7 +210,8 @@ __global__ void __launch_bounds__(128) plain_kernel(const __grid_constant__ DevS
   }
 }
 
-// CalculateDistance at n points (the reference's distance_engine.cl:42 job).
+// CalculateDistance at n points (the reference's distance_engine.cl:42 job),
+// one thread per point: extended and 4-D scenes, and sequences that blend.
 template <class T, int F, bool W, int V>
 __global__ void __launch_bounds__(128) distance_kernel(const __grid_constant__ DevScene sc, const double *pts,
                                                        long long n, double detail, int normal_mode, double *dist,
@@ -220,6 +223,68 @@ __global__ void __launch_bounds__(128) distance_kernel(const __grid_constant__ D
                                      normal_mode != 0, &it);
   dist[i] = double(d);
   if (iters) iters[i] = it;
+}
+
+// The same for scenes without the extended features, a warp at a time over
+// points of uneven orbit length: a warp owns every gridwide-strided group of
+// 32 points (neighbouring points tend to cost alike, so striding evens out the
+// warps), and a lane whose orbit has ended takes the warp's next point while
+// the others iterate on.  Points inside the set run maxN iterations (250 for
+// the default Mandelbulb) next to points that leave after two: with one thread
+// per point 4.2 of 32 lanes were active.  Bound by the FP64 pipe and the
+// packing of the last orbits; 1 M random points, FP64, one thread per point ->
+// this kernel: Mandelbulb 5989 -> 1623 us, Mandelbox 305 -> 161 us, Menger
+// sponge 59 -> 42 us.
+template <class T, int F, int V>
+__global__ void __launch_bounds__(128) distance_refill_kernel(const __grid_constant__ DevScene sc, const double *pts,
+                                                              long long n, double detail, int normal_mode,
+                                                              double *dist, int *iters, int idle) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long groups = (n + 31) / 32;
+  // the warp's points in its own order: q -> ((warp + (q / 32) * warps) * 32 + q % 32)
+  const long long mine = warp < groups ? ((groups - 1 - warp) / warps + 1) * 32 : 0;
+  const int maxN = sc.formula_maxiter * ((normal_mode && sc.iter_thresh) ? 5 : 1);
+  OrbitLane<T> e;
+  e.end = ORBIT_MAXITER;
+  bool has = false;
+  long long at = 0, next = 0;
+  for (;;) {
+    const unsigned need = __ballot_sync(FULL, !has);
+    if (need && next < mine) {
+      const long long q = next + __popc(need & ((1u << lane) - 1u));
+      next += __popc(need);
+      if (!has && q < mine) {
+        at = (warp + (q >> 5) * warps) * 32 + (q & 31);
+        if (at < n) {
+          orbit_begin(e, T(pts[3 * at]), T(pts[3 * at + 1]), T(pts[3 * at + 2]), maxN);
+          has = true;
+        }
+      }
+    }
+    if (!__any_sync(FULL, has)) {
+      if (next >= mine) break;
+      continue;
+    }
+    // iterate until enough lanes wait for a new point (the drained warp: until all have ended)
+    const int keep = next < mine ? 32 - idle : 0;
+    if (has && e.end == ORBIT_RUNS) {
+      do {
+        orbit_pass<T, F>(sc, e, maxN);
+      } while (e.end == ORBIT_RUNS && __popc(__ballot_sync(__activemask(), 1)) > keep);
+    }
+    __syncwarp();
+    if (has && e.end != ORBIT_RUNS) {
+      const V4<T> z{e.zx, e.zy, e.zz, T(0.0)};
+      const T d = final_distance<T, F, false>(sc, z, len4<T, false>(z), e.de);
+      const int it = e.end == ORBIT_MAXITER ? e.it + 1 : e.it;
+      dist[at] = double(distance_tail<T>(sc, d, it, e.end != ORBIT_BAILOUT, T(detail), normal_mode != 0));
+      if (iters) iters[at] = it;
+      has = false;
+    }
+  }
 }
 
 template <class T, class R, int V>
@@ -257,6 +322,8 @@ int launch_distance_t(const DevScene &sc, const double *pts, int64_t n, double d
   const dim3 grid(unsigned((n + 127) / 128));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool ext = scene_extended(sc);
+  bool blend = false;
+  for (int k = 0; k < sc.n; k++) blend = blend || sc.slot[k].d[P_WEIGHT] != 1.0;
   if (sc.has_w) {
     if constexpr (sizeof(T) == 8) {
       if (ext) distance_kernel<T, F_EXT, true, V><<<grid, block, 0, s>>>(sc, pts, n, detail, normal_mode, dist, iters);
@@ -266,8 +333,35 @@ int launch_distance_t(const DevScene &sc, const double *pts, int64_t n, double d
     }
   } else if (ext) {
     distance_kernel<T, F_EXT, false, V><<<grid, block, 0, s>>>(sc, pts, n, detail, normal_mode, dist, iters);
-  } else {
+  } else if (blend) {
     distance_kernel<T, 0, false, V><<<grid, block, 0, s>>>(sc, pts, n, detail, normal_mode, dist, iters);
+  } else {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // CTAs per SM and the waiting lanes that end a round, per formula, from a
+    // sweep over 4 k to 4 M points (1 M points, FP64, per CTAs 4/6/7/8): box
+    // 192/161/161/165 us, Menger 8: 42 us, sequence 8/16: 137/118 us.  A
+    // Mandelbulb pass costs more than a refill, so two waiting lanes end the
+    // round (idle 2/8/16: 1623/1881/2394 us), and a warp needs about 128
+    // points to pack the long orbits (131072 points, 32/64/128/256 per warp:
+    // 761/526/415/743 us) - unless that left a scheduler without a warp.
+    const long long all = (n + 31) / 32;
+    const auto blocks = [&](int ctas, long long warps) {
+      return dim3(unsigned((std::max<long long>(1, std::min<long long>(warps, 4ll * ctas * sms)) + 3) / 4));
+    };
+    const int F = sc.is_hybrid ? 0 : sc.uniform_formula;
+#define REFILL(FORMULA, GRID, IDLE) \
+  distance_refill_kernel<T, FORMULA, V><<<GRID, block, 0, s>>>(sc, pts, n, detail, normal_mode, dist, iters, IDLE)
+    switch (F) {
+      case MBR_FORMULA_MANDELBULB:
+        REFILL(MBR_FORMULA_MANDELBULB, blocks(6, std::max<long long>((n + 127) / 128, std::min<long long>(all, 4ll * sms))), 2);
+        break;
+      case MBR_FORMULA_MANDELBOX: REFILL(MBR_FORMULA_MANDELBOX, blocks(7, all), 16); break;
+      case MBR_FORMULA_MENGER_SPONGE: REFILL(MBR_FORMULA_MENGER_SPONGE, blocks(8, all), 16); break;
+      default: REFILL(0, blocks(16, all), 8); break;
+    }
+#undef REFILL
   }
   return int(cudaGetLastError());
 }
