@@ -223,7 +223,12 @@ __device__ __forceinline__ double fmadd(double a, double b, double c) { return f
 // iterations per estimate, so a vote every 12 is cheap against the wait it
 // causes (measured on the 1080p Mandelbox: 2 -> 7.5 ms, 6 -> 6.4 ms,
 // 12 -> 6.3 ms per frame), while the Mandelbulb's 1-3 iterations per
-// estimate at the usual views want a vote every 2.
+// estimate at the usual views want a vote every 2.  The iterations between
+// two votes are unrolled where one is a few dozen instructions; the
+// reference-order policy's iteration (kHyb: a dispatch over formulas, library
+// functions inlined) is not: four copies of it overran the instruction
+// caches, half of all stall samples (1080p x 16 spp hybrid GI 338.8 ->
+// 188.2 ms, an 800x600 frame with primitives 14.77 -> 8.59 ms).
 template <int FK>
 struct kVoteEvery {
   static constexpr int n = (FK == FK_BULB) ? 2 : ((FK == FK_ANY) ? 4 : 12);
@@ -614,7 +619,7 @@ __device__ __forceinline__ void run_stage(Stage &S, const typename P::Params &fp
     if (iterating) {
       for (;;) {
         bool ended = false;
-#pragma unroll
+#pragma unroll (P::kHyb ? 1 : kVoteEvery<FK>::n)
         for (int u = 0; u < kVoteEvery<FK>::n; u++) {
           if (!P::template step<FK>(kind, e, fp)) {
             ended = true;
