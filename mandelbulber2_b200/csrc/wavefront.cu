@@ -123,8 +123,10 @@ struct WideParams {
   double bailout;
   double jc[3];  // julia_c * fractal_constant_factor
   double cm[3];  // fractal_constant_factor
-  // simple Mandelbox: folding limit, fR2, fR2/mR2, scale, |scale|, bailout^2
-  double lim, fr2, fmx, scale, ascale, bailout2;
+  // simple Mandelbox: folding limit, fR2, fR2/mR2, scale, bailout^2, and the
+  // squared radii outside which the sphere fold's factor is fmx or 1 whatever
+  // the rounding of the reciprocal (2^-40 away from mR2 and fR2)
+  double lim, fr2, fmx, scale, bailout2, r2_inner, r2_outer;
   MbRot rot;  // Mandelbox rotations (the simple form is off when any is on)
 };
 
@@ -152,8 +154,9 @@ __host__ __device__ inline WideParams load_wide_params(const DevScene &sc) {
   w.fr2 = s.d[P_MB_FR2];
   w.fmx = F;
   w.scale = s.d[P_MB_SCALE];
-  w.ascale = s.d[P_MB_ABS_SCALE];
   w.bailout2 = w.bailout * w.bailout;
+  w.r2_inner = w.fr2 / w.fmx * (1.0 - 0x1p-40);
+  w.r2_outer = w.fr2 * (1.0 + 0x1p-40);
   return w;
 }
 
@@ -228,7 +231,8 @@ __device__ __forceinline__ double fmadd(double a, double b, double c) { return f
 // reference-order policy's iteration (kHyb: a dispatch over formulas, library
 // functions inlined) is not: four copies of it overran the instruction
 // caches, half of all stall samples (1080p x 16 spp hybrid GI 338.8 ->
-// 188.2 ms, an 800x600 frame with primitives 14.77 -> 8.59 ms).
+// 188.2 ms, an 800x600 frame with primitives 14.77 -> 8.59 ms); the FP64
+// Mandelbox is by four (12: 33.8 ms on the 1080p deep zoom, 2 to 6: 31.4 ms).
 template <int FK>
 struct kVoteEvery {
   static constexpr int n = (FK == FK_BULB) ? 2 : ((FK == FK_ANY) ? 4 : 12);
@@ -262,6 +266,7 @@ struct Prec32 {
   __host__ __device__ static int kind(const Params &f) { return fast_kind(f); }
   __device__ static const Params &job_params(const Launch &L, int job) { return L.fps[job]; }
 
+  template <int FK>
   __device__ static void start(State &e, const Params &fp, float qx, float qy, float qz) {
     e.z.x = qx;
     e.z.y = qy;
@@ -273,8 +278,9 @@ struct Prec32 {
     e.it = 0;
     e.r2 = fmaf(qx, qx, fmaf(qy, qy, qz * qz));
   }
+  template <int FK>
   __device__ static void start(State &e, const Params &fp, double qx, double qy, double qz) {
-    start(e, fp, float(qx), float(qy), float(qz));
+    start<FK>(e, fp, float(qx), float(qy), float(qz));
   }
 
   // One iteration; false once the orbit is done (bailout or maxN).
@@ -290,11 +296,18 @@ struct Prec32 {
     return e.r2 <= fp.bailout2 && e.it < fp.maxN;
   }
 
+  template <int FK>
   __device__ static float distance(const State &e, const Params &fp, float detail, int &iters) {
     iters = (e.r2 > fp.bailout2) ? e.it : e.it + 1;
     return final_de(fp, e.r2, e.dr, iters, detail);
   }
 };
+
+// 2 clamp(z, -L, L) - z, for |z| > L the rounded 2L - z or -2L - z, else z itself
+__device__ __forceinline__ double box_fold(double z, double L) {
+  const double w = copysign(2.0 * L, z) - z;
+  return fabs(z) > L ? w : z;
+}
 
 struct Prec64 {
   typedef double D;
@@ -307,11 +320,23 @@ struct Prec64 {
   __host__ __device__ static int kind(const Params &w) { return wide_kind(w); }
   __device__ static const Params &job_params(const Launch &L, int job) { return L.wps[job]; }
 
-  // Compute's start (compute_fractal.cpp:74-130): z = c = the point, DE = 1
-  __device__ static void start(State &e, const Params &, double qx, double qy, double qz) {
+  // Compute's start (compute_fractal.cpp:74-130): z = c = the point, DE = 1.
+  // The simple Mandelbox keeps what is added to every pass in place of c.
+  template <int FK>
+  __device__ static void start(State &e, const Params &fp, double qx, double qy, double qz) {
     e.zx = qx;
     e.zy = qy;
     e.zz = qz;
+    if (FK == FK_BOX_SIMPLE) {
+      e.cx = !fp.add_c ? 0.0 : (fp.julia ? fp.jc[0] : qx * fp.cm[0]);
+      e.cy = !fp.add_c ? 0.0 : (fp.julia ? fp.jc[1] : qy * fp.cm[1]);
+      e.cz = !fp.add_c ? 0.0 : (fp.julia ? fp.jc[2] : qz * fp.cm[2]);
+      e.dr = 1.0;
+      e.r = fma(qx, qx, fma(qy, qy, qz * qz));
+      e.it = 0;
+      e.brk = 0;
+      return;
+    }
     e.cx = qx;
     e.cy = qy;
     e.cz = qz;
@@ -328,46 +353,38 @@ struct Prec64 {
   // sphere-fold factor clamp(fR2 / r2, 1, fR2 / mR2) with a correctly rounded
   // reciprocal, scale and c-addition fused, bailout tested on |z|^2 and |z|
   // taken once when the orbit ends; the result differs from the reference's
-  // operation order in the last bits only.
+  // operation order in the last bits only.  The FP64 minimum and maximum are
+  // several instructions each, so the folds are a compare and a select, and
+  // the reciprocal is taken only between the radii (with the fold as minimum
+  // and maximum and the reciprocal in every pass: 86 instead of about 50
+  // instructions a pass; the 1080p deep zoom 57.9 -> 28.4 ms, a stage-S tail of
+  // orbits that never leave 96 -> 66 ms.  With the reciprocal in every pass
+  // 32.2 ms; two passes per bailout test, the second speculative, 30.5 ms).
   template <int FK>
   __device__ static bool step(int kind, State &e, const Params &fp) {
     const int k = (FK == FK_ANY) ? kind : FK;
     if (k == FK_BOX_SIMPLE) {
       const double L = fp.lim;
-      const double x = fma(2.0, fmin(fmax(e.zx, -L), L), -e.zx);
-      const double y = fma(2.0, fmin(fmax(e.zy, -L), L), -e.zy);
-      const double z = fma(2.0, fmin(fmax(e.zz, -L), L), -e.zz);
+      const double x = box_fold(e.zx, L), y = box_fold(e.zy, L), z = box_fold(e.zz, L);
       const double r2 = fma(x, x, fma(y, y, z * z));
-      const double fs = fmin(fmax(fp.fr2 * __drcp_rn(r2), 1.0), fp.fmx);
-      const double s = fs * fp.scale;
-      e.dr = fma(e.dr, fs * fp.ascale, 1.0);
-      double ax = 0.0, ay = 0.0, az = 0.0;
-      if (fp.add_c) {
-        if (fp.julia) {
-          ax = fp.jc[0];
-          ay = fp.jc[1];
-          az = fp.jc[2];
-        } else {
-          ax = e.cx * fp.cm[0];
-          ay = e.cy * fp.cm[1];
-          az = e.cz * fp.cm[2];
-        }
+      double fs = r2 <= fp.r2_inner ? fp.fmx : 1.0;
+      if (r2 > fp.r2_inner && r2 < fp.r2_outer) {
+        fs = fp.fr2 * __drcp_rn(r2);
+        fs = fs < 1.0 ? 1.0 : fs;
+        fs = fs > fp.fmx ? fp.fmx : fs;
       }
-      e.zx = fma(x, s, ax);
-      e.zy = fma(y, s, ay);
-      e.zz = fma(z, s, az);
+      const double s = fs * fp.scale;
+      e.dr = fma(e.dr, fabs(s), 1.0);  // fs > 0: |fs scale| is fs |scale|
+      e.zx = fma(x, s, e.cx);
+      e.zy = fma(y, s, e.cy);
+      e.zz = fma(z, s, e.cz);
       e.it++;
-      const double rr = fma(e.zx, e.zx, fma(e.zy, e.zy, e.zz * e.zz));
-      if (!(rr <= fp.bailout2) && fp.check_bailout) {
-        e.r = sqrt(rr);
+      e.r = fma(e.zx, e.zx, fma(e.zy, e.zy, e.zz * e.zz));  // |z|^2: distance() takes the root
+      if (!(e.r <= fp.bailout2)) {  // a single formula always checks its bailout
         e.brk = 1;
         return false;
       }
-      if (e.it >= fp.maxN) {
-        e.r = sqrt(rr);
-        return false;
-      }
-      return true;
+      return e.it < fp.maxN;
     }
     V4<double> z{e.zx, e.zy, e.zz, 0.0};
     const V4<double> last = z;
@@ -409,9 +426,10 @@ struct Prec64 {
 
   // Final DE and CalculateDistanceSimple's clamps (compute_fractal.cpp:561-621,
   // calculate_distance.cpp:569, 604-605).
+  template <int FK>
   __device__ static double distance(const State &e, const Params &fp, double detail, int &iters) {
     iters = e.brk ? e.it : e.it + 1;
-    const double r = e.r, DE = e.dr;
+    const double r = FK == FK_BOX_SIMPLE ? sqrt(e.r) : e.r, DE = e.dr;
     double d;
     if (DE > 0.0) {
       if (fp.de_fn == 2) d = (r > 1.0) ? 0.5 * r * log(r) / DE : 0.0;
@@ -451,6 +469,7 @@ struct PrecHybT {
   };
   __host__ __device__ static int kind(const Params &) { return FK_ANY; }
 
+  template <int FK>
   __device__ static void start(State &e, const Params &, float qx, float qy, float qz) {
     e.zx = qx;
     e.zy = qy;
@@ -463,8 +482,9 @@ struct PrecHybT {
     e.it = 0;
     e.brk = 0;
   }
+  template <int FK>
   __device__ static void start(State &e, const Params &fp, double qx, double qy, double qz) {
-    start(e, fp, float(qx), float(qy), float(qz));
+    start<FK>(e, fp, float(qx), float(qy), float(qz));
   }
 
   template <int FK>
@@ -522,6 +542,7 @@ struct PrecHybT {
     return e.it < sc.formula_maxiter;
   }
 
+  template <int FK>
   __device__ static float distance(const State &e, const Params &fp, float detail, int &iters) {
     const DevScene &sc = *fp.sc;
     if (EXT && sc.limits) {  // outside the limit box: its distance (the iteration is not used)
@@ -600,7 +621,7 @@ __device__ __forceinline__ void run_stage(Stage &S, const typename P::Params &fp
       if (((need >> lane) & 1u) && rank < take) {
         typename Stage::Real qx, qy, qz;
         if (S.start(q_next + rank, qx, qy, qz)) {
-          P::start(e, Stage::kMulti ? S.params() : fpk, qx, qy, qz);
+          P::template start<FK>(e, Stage::kMulti ? S.params() : fpk, qx, qy, qz);
           has = true;
           iterating = true;
         }
@@ -619,7 +640,7 @@ __device__ __forceinline__ void run_stage(Stage &S, const typename P::Params &fp
     if (iterating) {
       for (;;) {
         bool ended = false;
-#pragma unroll (P::kHyb ? 1 : kVoteEvery<FK>::n)
+#pragma unroll (P::kHyb ? 1 : (P::kWide && FK == FK_BOX_SIMPLE ? 4 : kVoteEvery<FK>::n))
         for (int u = 0; u < kVoteEvery<FK>::n; u++) {
           if (!P::template step<FK>(kind, e, fp)) {
             ended = true;
@@ -637,12 +658,12 @@ __device__ __forceinline__ void run_stage(Stage &S, const typename P::Params &fp
     // ---- lanes whose estimate is done: distance, then the march step
     if (has && !iterating) {
       int iters;
-      const typename P::D d = P::distance(e, fp, S.detail(), iters);
+      const typename P::D d = P::template distance<FK>(e, fp, S.detail(), iters);
       de_n++;
       it_n += (unsigned long long)iters;
       typename Stage::Real qx, qy, qz;
       if (S.step(d, iters, qx, qy, qz)) {
-        P::start(e, Stage::kMulti ? S.params() : fpk, qx, qy, qz);
+        P::template start<FK>(e, Stage::kMulti ? S.params() : fpk, qx, qy, qz);
         iterating = true;
       } else {
         has = false;
@@ -672,6 +693,19 @@ __device__ __forceinline__ void flush_counts(const DevOutputs &out, unsigned int
     if (it) atomicAdd(st + K_ITERS, it);
   }
 }
+
+// Blocks of 256 per SM that a stage's registers have to leave room for.  The
+// FP64 Mandelbox trades registers for warps (1080p deep zoom, stage P at
+// 128 / 85 / 64 registers 3.14 / 2.87 / 2.74 ms, stage S 24.8 / 24.1 / 24.2 ms);
+// its batch form holds the job's parameters in registers too, and stage S ends
+// in a tail of single long orbits, which spills would lengthen (P 82 / 78 ms,
+// S 67 / 82 ms at 128 / 85).
+template <int FK, bool MULTI, class P>
+struct kMinBlocks {
+  static constexpr bool box64 = P::kWide && FK == FK_BOX_SIMPLE;
+  static constexpr int primary = box64 ? (MULTI ? 3 : 4) : 0;  // 0: none asked
+  static constexpr int shade = box64 ? (MULTI ? 2 : 3) : 0;
+};
 
 // ============================================================================
 // Stage P: primary march with binary refinement, one task per pixel.
@@ -926,7 +960,7 @@ struct PrimaryStage {
 };
 
 template <int FK, bool MULTI, class P>
-__global__ void __launch_bounds__(256) primary_kernel(const __grid_constant__ DevFrame fr,
+__global__ void __launch_bounds__(256, kMinBlocks<FK, MULTI, P>::primary) primary_kernel(const __grid_constant__ DevFrame fr,
                                                       const __grid_constant__ typename P::Params fp0,
                                                       const __grid_constant__ WJob job0,
                                                       const __grid_constant__ Launch L, DevOutputs out) {
@@ -1343,7 +1377,7 @@ __device__ __forceinline__ void shade_body(const DevFrame &fr, const typename P:
 }
 
 template <int FK, bool MULTI, class P>
-__global__ void __launch_bounds__(256) shade_kernel(const __grid_constant__ DevFrame fr,
+__global__ void __launch_bounds__(256, kMinBlocks<FK, MULTI, P>::shade) shade_kernel(const __grid_constant__ DevFrame fr,
                                                     const __grid_constant__ typename P::Params fp0,
                                                     const __grid_constant__ Launch L, DevOutputs out) {
   shade_body<FK, MULTI, P, false>(fr, fp0, L, out);
@@ -1935,7 +1969,7 @@ static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const 
         Lp.hits = lists[0];
 #define GP_LAUNCH(K) \
   case K:            \
-    if constexpr (!P::kHyb || K == FK_ANY) gi_primary_kernel<K, P><<<grid, block, 0, st>>>(fr, fp0, j0, Lp, out); \
+    if constexpr (P::kHyb == (K == FK_ANY)) gi_primary_kernel<K, P><<<grid, block, 0, st>>>(fr, fp0, j0, Lp, out); \
     break;
         GI_CASES(GP_LAUNCH)
 #undef GP_LAUNCH
@@ -1950,7 +1984,7 @@ static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const 
         Lb.normal_slot = K_GI;
 #define GV_LAUNCH(K)                                                                                   \
   case K:                                                                                              \
-    if constexpr (!P::kHyb || K == FK_ANY) {                                                           \
+    if constexpr (P::kHyb == (K == FK_ANY)) {                                                           \
       normal_kernel<K, false, P><<<grid, block, 0, st>>>(fr, fp0, Lb, out);                             \
       gi_vertex_kernel<K, P><<<grid, block, 0, st>>>(fr, fp0, Lb, out);                                 \
     }                                                                                                  \
@@ -1966,7 +2000,7 @@ static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const 
   }
 #define STAGE_LAUNCH(KERNEL, K, ...)                                                    \
   case K:                                                                               \
-    if constexpr (!P::kHyb || K == FK_ANY) KERNEL<K, MULTI, P><<<grid, block, 0, st>>>(__VA_ARGS__); \
+    if constexpr (P::kHyb == (K == FK_ANY)) KERNEL<K, MULTI, P><<<grid, block, 0, st>>>(__VA_ARGS__); \
     break;
 #define STAGE(KERNEL, ...)                                                              \
   switch (fk) {                                                                         \
