@@ -34,6 +34,10 @@ UNITS = [
     ("plain_fp64_strict.cu", ["--fmad=false"]),
     ("plain_mixed.cu", []),
     ("wavefront.cu", []),
+    ("wavefront32.cu", []),
+    ("wavefront64.cu", []),
+    ("wavefront_batch.cu", []),
+    ("wavefront_hybrid.cu", []),
     ("probe.cu", []),
     ("adjoint.cu", []),
 ]

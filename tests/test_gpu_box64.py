@@ -1,4 +1,4 @@
-"""The FP64 wavefront's Mandelbox iteration (csrc/wavefront.cu, Prec64) where
+"""The FP64 wavefront's Mandelbox iteration (csrc/wavefront.cuh, Prec64) where
 its folds branch: a tiny minimum radius (a large sphere-fold factor),
 radii that lie close together, a positive scale, a Julia constant, c left out.
 Held to the FP64 wavefront's bars against the oracle: hits and iteration counts
