@@ -32,6 +32,10 @@ UNITS = [
     ("fract_loader.cpp", []),
     ("plain_fp64.cu", []),
     ("plain_fp64_strict.cu", ["--fmad=false"]),
+    ("staged_fp64.cu", []),
+    ("staged_fp64_strict.cu", ["--fmad=false"]),
+    ("staged_keyed_fp64.cu", []),
+    ("staged_keyed_fp64_strict.cu", ["--fmad=false"]),
     ("plain_mixed.cu", []),
     ("wavefront.cu", []),
     ("wavefront32.cu", []),

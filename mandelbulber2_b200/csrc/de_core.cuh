@@ -342,7 +342,7 @@ __device__ __forceinline__ T sgn_of(T v) {
 // computed.  pk: aux.pseudoKleinianDE, which the pseudo-Kleinian DE function
 // reads.
 template <class T>
-__device__ __noinline__ void f_pseudo_kleinian(V4<T> &z, T &DE, T &pk, const DevSlot &s, int i) {
+__device__ __forceinline__ void f_pseudo_kleinian(V4<T> &z, T &DE, T &pk, const DevSlot &s, int i) {
   const double *x = s.x;
   if (x[PKX_SPH_INV] != 0.0 && i >= int(x[PKX_START_X]) && i < int(x[PKX_STOP_1])) {  // :33-44
     z.x = z.x + T(x[PKX_OFFSET000]);
@@ -433,7 +433,7 @@ __device__ __noinline__ void f_pseudo_kleinian(V4<T> &z, T &DE, T &pk, const Dev
 // power-2 bulb with its z factor; a delta-DE formula (its analytic DE terms
 // apply only under a forced analytic method)
 template <class T>
-__device__ __noinline__ void f_box_fold_bulb_pow2(V4<T> &z, T r, T &DE, const DevSlot &s) {
+__device__ __forceinline__ void f_box_fold_bulb_pow2(V4<T> &z, T r, T &DE, const DevSlot &s) {
   const double *x = s.x;
   const double ff = x[BFX_FOLD];
   if (m_abs(z.x) > T(ff)) z.x = T(double(sgn_of(z.x)) * ff * 2.0) - z.x;
@@ -477,7 +477,7 @@ __device__ __noinline__ void f_box_fold_bulb_pow2(V4<T> &z, T r, T &DE, const De
 // that may vary from one iteration to the next (scaleA = aux.actualScaleA),
 // the power-2 bulb with its z factor
 template <class T>
-__device__ __noinline__ void f_box_fold_bulb_pow2_v2(V4<T> &z, T &DE, T &scaleA, const DevSlot &s, int i) {
+__device__ __forceinline__ void f_box_fold_bulb_pow2_v2(V4<T> &z, T &DE, T &scaleA, const DevSlot &s, int i) {
   const double *x = s.x;
   if (i >= int(x[B2X_START_B]) && i < int(x[B2X_STOP_B])) {  // tglad fold :35-45
     const T ax = T(x[B2X_ADD111]), ay = T(x[B2X_ADD111 + 1]), az = T(x[B2X_ADD111 + 2]);
@@ -549,7 +549,7 @@ __device__ __noinline__ void f_box_fold_bulb_pow2_v2(V4<T> &z, T &DE, T &scaleA,
 // a curve over the iterations, scale, offset, c-addition (optionally of aux.c
 // permuted every iteration), rotation and a tweak scale.  c: aux.const_c.
 template <class T>
-__device__ __noinline__ void f_abox_mod11(V4<T> &z, T &DE, AuxX<T> &ax, const V4<T> &c, const DevSlot &s, int i) {
+__device__ __forceinline__ void f_abox_mod11(V4<T> &z, T &DE, AuxX<T> &ax, const V4<T> &c, const DevSlot &s, int i) {
   const double *x = s.x;
   ax.scale = T(x[ABX_MB_SCALE] + x[ABX_SCALE_VARY] * (fabs(double(ax.scale)) - 1.0));  // :36-37
   if (i >= int(x[ABX_START_B]) && i < int(x[ABX_STOP_B])) {  // tglad fold :41-55
@@ -638,7 +638,7 @@ __device__ __noinline__ void f_abox_mod11(V4<T> &z, T &DE, AuxX<T> &ax, const V4
 // 29-145) without the aux.color terms; pk and pos_neg are
 // aux.pseudoKleinianDE and aux.pos_neg
 template <class T>
-__device__ __noinline__ void f_pseudo_kleinian_mod4(V4<T> &z, T &DE, AuxX<T> &ax, const DevSlot &s, int i) {
+__device__ __forceinline__ void f_pseudo_kleinian_mod4(V4<T> &z, T &DE, AuxX<T> &ax, const DevSlot &s, int i) {
   const double *x = s.x;
   if (x[P4X_SPH_INV] != 0.0 && i >= int(x[P4X_START_X]) && i < int(x[P4X_STOP_1])) {  // :37-47
     z.x = z.x + T(x[P4X_OFFSET000]);
@@ -746,7 +746,7 @@ __device__ __forceinline__ V4<T> benesi_out(const V4<T> &z) {
 // T1 mod, an abs fold, a Menger fold, the Kleinian fold (two variants) and
 // the custom distance aux.dist (ax.dist)
 template <class T>
-__device__ __noinline__ void f_pseudo_kleinian_std_de(V4<T> &z, T &DE, AuxX<T> &ax, const DevSlot &s, int i) {
+__device__ __forceinline__ void f_pseudo_kleinian_std_de(V4<T> &z, T &DE, AuxX<T> &ax, const DevSlot &s, int i) {
   const double *x = s.x;
   if (x[PSX_P_ON] != 0.0 && i >= int(x[PSX_START_P]) && i < int(x[PSX_STOP_P1])) {  // prism :38-58
     z.y = m_abs(z.y);
@@ -910,7 +910,7 @@ __device__ __forceinline__ T g3dot(const G3<T> &a, const G3<T> &b) {
 // polyhedron (mirror, rotation line or inversion point, above the melt
 // layer), then the Mandelbox sphere fold, main rotation and scale
 template <class T>
-__device__ __noinline__ void f_generalized_fold_box(V4<T> &z, T &DE, const DevSlot &s) {
+__device__ __forceinline__ void f_generalized_fold_box(V4<T> &z, T &DE, const DevSlot &s) {
   const double *x = s.x;
   const int sides = int(x[GFX_SIDES]);
   const T solid = T(x[GFX_SOLID]), melt = T(x[GFX_MELT]);
@@ -1016,7 +1016,7 @@ __device__ __noinline__ void f_generalized_fold_box(V4<T> &z, T &DE, const DevSl
 // a Mandelbulb with optional pre-folds, acos latitude, sin/cos swap, polar
 // scalings and a y fold; dist is aux.dist (set when its own DE block is on)
 template <class T>
-__device__ __noinline__ void f_mandelbulb_pupuku(V4<T> &z, T r, T &DE, T &dist, const DevSlot &s, int i) {
+__device__ __forceinline__ void f_mandelbulb_pupuku(V4<T> &z, T r, T &DE, T &dist, const DevSlot &s, int i) {
   const double *x = s.x;
   if (x[PPX_P_ON] != 0.0 && i >= int(x[PPX_START_P]) && i < int(x[PPX_STOP_P])) {  // :34-45
     if (x[PPX_CX] != 0.0) z.x = m_abs(z.x);
@@ -1094,7 +1094,7 @@ __device__ __noinline__ void f_mandelbulb_pupuku(V4<T> &z, T r, T &DE, T &dist, 
 // custom-DE formula) after sphere inversion, a tiling fold, a varying scale
 // (scaleA = aux.actualScaleA), offset and rotation
 template <class T>
-__device__ __noinline__ void f_difs_hextgrid2(V4<T> &z, T &DE, AuxX<T> &ax, const DevSlot &s, int i) {
+__device__ __forceinline__ void f_difs_hextgrid2(V4<T> &z, T &DE, AuxX<T> &ax, const DevSlot &s, int i) {
   const double *x = s.x;
   if (x[HGX_SPH_INV] != 0.0 && i >= int(x[HGX_START_X]) && i < int(x[HGX_STOP_1])) {  // :35-45
     z.x = z.x + T(x[HGX_OFFSET000]);
@@ -1159,7 +1159,7 @@ __device__ __noinline__ void f_difs_hextgrid2(V4<T> &z, T &DE, AuxX<T> &ax, cons
 // cFractalMengerMod1::FormulaCode (fractal_menger_mod1.cpp:29-103), the
 // aux.color terms left out
 template <class T>
-__device__ __noinline__ void f_menger_mod1(V4<T> &z, T &DE, const DevSlot &s, int i) {
+__device__ __forceinline__ void f_menger_mod1(V4<T> &z, T &DE, const DevSlot &s, int i) {
   const double *x = s.x;
   z = V4<T>{m_abs(z.x), m_abs(z.y), m_abs(z.z), m_abs(z.w)};
   T t;
@@ -1267,6 +1267,26 @@ __device__ __forceinline__ void f_ifs(V4<T> &z, T &DE, const IfsBlock &b) {
   DE = DE * m_abs(sc);
 }
 
+// One step of a formula by settings key, the formula known at compile time.
+template <class T, int FORMULA>
+__device__ __forceinline__ void keyed_formula(V4<T> &z, T r, T &DE, const DevSlot &s, int i, const V4<T> &c, AuxX<T> &ax) {
+  if constexpr (FORMULA == MBR_FORMULA_PSEUDO_KLEINIAN) f_pseudo_kleinian<T>(z, DE, ax.pk, s, i);
+  else if constexpr (FORMULA == MBR_FORMULA_BOX_FOLD_BULB_POW2) f_box_fold_bulb_pow2<T>(z, r, DE, s);
+  else if constexpr (FORMULA == MBR_FORMULA_BOX_FOLD_BULB_POW2_V2) f_box_fold_bulb_pow2_v2<T>(z, DE, ax.scaleA, s, i);
+  else if constexpr (FORMULA == MBR_FORMULA_ABOX_MOD11) f_abox_mod11<T>(z, DE, ax, c, s, i);
+  else if constexpr (FORMULA == MBR_FORMULA_PSEUDO_KLEINIAN_MOD4) f_pseudo_kleinian_mod4<T>(z, DE, ax, s, i);
+  else if constexpr (FORMULA == MBR_FORMULA_PSEUDO_KLEINIAN_STD_DE) f_pseudo_kleinian_std_de<T>(z, DE, ax, s, i);
+  else if constexpr (FORMULA == MBR_FORMULA_GENERALIZED_FOLD_BOX) f_generalized_fold_box<T>(z, DE, s);
+  else if constexpr (FORMULA == MBR_FORMULA_MANDELBULB_PUPUKU) f_mandelbulb_pupuku<T>(z, r, DE, ax.dist, s, i);
+  else if constexpr (FORMULA == MBR_FORMULA_DIFS_HEXTGRID2) f_difs_hextgrid2<T>(z, DE, ax, s, i);
+  else if constexpr (FORMULA == MBR_FORMULA_MENGER_MOD1) f_menger_mod1<T>(z, DE, s, i);
+}
+// The same as a called function, for the kernels that carry every formula.
+template <class T, int FORMULA>
+__device__ __noinline__ void keyed_call(V4<T> &z, T r, T &DE, const DevSlot &s, int i, const V4<T> &c, AuxX<T> &ax) {
+  keyed_formula<T, FORMULA>(z, r, DE, s, i, c, ax);
+}
+
 // EXT: the formulas beyond the three specialised ones and the Mandelbox
 // rotations are compiled in; kernels of scenes that use none of them (hybrids
 // of the three included) are built without that code.
@@ -1278,16 +1298,16 @@ __device__ __forceinline__ void formula_dispatch(int formula, V4<T> &z, T r, T &
                                                  AuxX<T> &ax) {
   if constexpr (EXT) {
     switch (formula) {
-      case MBR_FORMULA_PSEUDO_KLEINIAN: f_pseudo_kleinian<T>(z, DE, ax.pk, s, i); break;
-      case MBR_FORMULA_BOX_FOLD_BULB_POW2_V2: f_box_fold_bulb_pow2_v2<T>(z, DE, ax.scaleA, s, i); break;
-      case MBR_FORMULA_ABOX_MOD11: f_abox_mod11<T>(z, DE, ax, c, s, i); break;
-      case MBR_FORMULA_PSEUDO_KLEINIAN_MOD4: f_pseudo_kleinian_mod4<T>(z, DE, ax, s, i); break;
-      case MBR_FORMULA_PSEUDO_KLEINIAN_STD_DE: f_pseudo_kleinian_std_de<T>(z, DE, ax, s, i); break;
-      case MBR_FORMULA_GENERALIZED_FOLD_BOX: f_generalized_fold_box<T>(z, DE, s); break;
-      case MBR_FORMULA_MANDELBULB_PUPUKU: f_mandelbulb_pupuku<T>(z, r, DE, ax.dist, s, i); break;
-      case MBR_FORMULA_DIFS_HEXTGRID2: f_difs_hextgrid2<T>(z, DE, ax, s, i); break;
-      case MBR_FORMULA_BOX_FOLD_BULB_POW2: f_box_fold_bulb_pow2<T>(z, r, DE, s); break;
-      case MBR_FORMULA_MENGER_MOD1: f_menger_mod1<T>(z, DE, s, i); break;
+      case MBR_FORMULA_PSEUDO_KLEINIAN: keyed_call<T, MBR_FORMULA_PSEUDO_KLEINIAN>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_BOX_FOLD_BULB_POW2_V2: keyed_call<T, MBR_FORMULA_BOX_FOLD_BULB_POW2_V2>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_ABOX_MOD11: keyed_call<T, MBR_FORMULA_ABOX_MOD11>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_PSEUDO_KLEINIAN_MOD4: keyed_call<T, MBR_FORMULA_PSEUDO_KLEINIAN_MOD4>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_PSEUDO_KLEINIAN_STD_DE: keyed_call<T, MBR_FORMULA_PSEUDO_KLEINIAN_STD_DE>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_GENERALIZED_FOLD_BOX: keyed_call<T, MBR_FORMULA_GENERALIZED_FOLD_BOX>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_MANDELBULB_PUPUKU: keyed_call<T, MBR_FORMULA_MANDELBULB_PUPUKU>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_DIFS_HEXTGRID2: keyed_call<T, MBR_FORMULA_DIFS_HEXTGRID2>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_BOX_FOLD_BULB_POW2: keyed_call<T, MBR_FORMULA_BOX_FOLD_BULB_POW2>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_MENGER_MOD1: keyed_call<T, MBR_FORMULA_MENGER_MOD1>(z, r, DE, s, i, c, ax); break;
       case MBR_FORMULA_QUATERNION: f_quaternion<T>(z, r, DE); break;
       case MBR_FORMULA_AEXION: f_aexion<T>(z, r, DE, s, i, c); break;
       case MBR_FORMULA_MANDELBULB: f_mandelbulb<T>(z, r, DE, s); break;
@@ -1545,7 +1565,7 @@ __device__ __forceinline__ int compute_orbit(const DevScene &sc, T px, T py, T p
   r = len4<T, W>(z);
   DE = T(1.0);
   AuxX<T> ax{T(1.0), T(0.0), T(0.0), T(1.0), T(1000.0), z};
-  if (F == F_EXT)  // aux.actualScale: the Mandelbox scale of the sequence's first slot (compute_fractal.cpp:97-98, 123)
+  if (F < 0)  // aux.actualScale: the Mandelbox scale of the sequence's first slot (compute_fractal.cpp:97-98, 123)
     ax.scale = T(sc.slot[TREE ? nd->slot : int(sc.seq[0])].d[P_MB_SCALE]);
   V4<T> lastZ{T(0.0), T(0.0), T(0.0), T(0.0)}, lastLastZ = lastZ;
   maxiter = true;
@@ -1553,7 +1573,7 @@ __device__ __forceinline__ int compute_orbit(const DevScene &sc, T px, T py, T p
   for (i = 0; i < maxN; i++) {
     lastLastZ = lastZ;
     lastZ = z;
-    const int k = TREE ? nd->slot : ((F > 0) ? 0 : ((i < sc.length) ? int(sc.seq[i]) : int(sc.seq[0])));
+    const int k = TREE ? nd->slot : ((F > 0 || F < F_EXT) ? 0 : ((i < sc.length) ? int(sc.seq[i]) : int(sc.seq[0])));
     const DevSlot &s = sc.slot[k];
     if (F == F_EXT) global_folds<T, W>(sc, z, r, DE);
     const V4<T> tempZ = z;
@@ -1562,6 +1582,8 @@ __device__ __forceinline__ int compute_orbit(const DevScene &sc, T px, T py, T p
       if (F == MBR_FORMULA_MANDELBULB) f_mandelbulb<T>(z, r, DE, s);
       if (F == MBR_FORMULA_MANDELBOX) f_mandelbox<T, W>(z, DE, s);
       if (F == MBR_FORMULA_MENGER_SPONGE) f_menger<T, W>(z, DE, s);
+    } else if (F < F_EXT) {
+      keyed_formula<T, -F>(z, r, DE, s, i, c, ax);
     } else if (s.d[P_WEIGHT] > 0.0) {
       formula_dispatch<T, W, F == F_EXT>(s.formula, z, r, DE, s, &sc.mbrot, &sc.ifs, i, c, ax);
     }
@@ -1577,7 +1599,7 @@ __device__ __forceinline__ int compute_orbit(const DevScene &sc, T px, T py, T p
         if (W) z.w = z.w + c.w;
       }
     }
-    if (!TREE && F <= 0 && sc.is_hybrid) {
+    if (!TREE && F <= 0 && F >= F_EXT && sc.is_hybrid) {
       const double kw = s.d[P_WEIGHT];
       if (kw < 1.0) {
         z = smooth4<T, W>(tempZ, z, kw);
@@ -1597,7 +1619,7 @@ __device__ __forceinline__ int compute_orbit(const DevScene &sc, T px, T py, T p
     }
     // the convergence bailout of pseudo- and Jos-Kleinian formulas
     // (compute_fractal.cpp:323-336; hybrid_fractal_sequences.cpp:242-246)
-    if (F == F_EXT && s.check_bailout && s.add_bail) {
+    if (F < 0 && s.check_bailout && s.add_bail) {
       maxiter = false;
       const T lim = T(0.1 / s.d[P_BAILOUT]);
       if (len4<T, W>(V4<T>{z.x - lastZ.x, z.y - lastZ.y, z.z - lastZ.z, z.w - lastZ.w}) / r < lim) break;
@@ -1706,7 +1728,7 @@ template <class T, int F, bool W>
 __device__ __forceinline__ T final_distance(const DevScene &sc, const V4<T> &z, T r, T DE, int de_final = -1,
                                             T pk = T(1.0), T dist = T(1000.0)) {
   if (!(DE > T(0.0))) return r;
-  if (F == F_EXT) {
+  if (F < 0) {
     switch (de_final >= 0 ? de_final : sc.de_final) {
       case DEF_LINEAR_OFFSET: return (r - (sizeof(T) == 8 ? T(sc.linear_de_offset) : T(sc.flinear_de_offset))) / DE;
       case DEF_LOG: return (r > T(1.0)) ? T(T(0.5) * r * m_log(r) / DE) : T(0.0);

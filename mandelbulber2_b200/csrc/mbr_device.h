@@ -7,6 +7,7 @@
 // It is passed to the kernels by value (__grid_constant__), so every lane
 // reads it through the constant cache.
 #pragma once
+#include <stddef.h>
 #include <stdint.h>
 
 #include "../../include/mbr.h"
@@ -296,6 +297,11 @@ struct Counters {
 // Plain per-pixel kernels: rows [0, height) of the frame.
 int launch_plain_fp64(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *stream);
 int launch_plain_fp64_strict(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *stream);
+// The same frames by stages (staged_plain.cuh): the scratch bytes a frame
+// needs, 0 where the per-pixel kernels render it, and the launch.
+size_t staged_plain_scratch(const DevScene &sc, const DevFrame &fr, bool strict);
+int launch_staged_fp64(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *scratch, void *stream);
+int launch_staged_fp64_strict(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *scratch, void *stream);
 int launch_plain_mixed(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *stream);
 int launch_distance_fp64(const DevScene &sc, const double *pts, int64_t n, double detail, int normal_mode,
                          double *dist, int32_t *iters, void *stream);

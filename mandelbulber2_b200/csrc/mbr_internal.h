@@ -27,6 +27,9 @@ mbr_status ctx_work(mbr_ctx *ctx, size_t words, unsigned long long **out);
 // Device buffer of the adjoint's per-block partial sums, grown on demand.
 mbr_status ctx_adjoint_partials(mbr_ctx *ctx, size_t bytes, double **out);
 
+// Gives back a context's hold on its device's frame pool.
+void frame_pool_release(int device);
+
 // wavefront.cu
 mbr_status render_wavefront(mbr_ctx *ctx, const DevScene &sc, const DevFrame &fr, const DevOutputs &out, int engine,
                             void *stream);

@@ -249,7 +249,7 @@ struct Prec32 {
   typedef Prec32 Normal;  // the policy of the normal stage
   typedef float D;  // distance and threshold arithmetic of the march
   typedef FastParams Params;
-  enum { kWide = 0, kHyb = 0, kGI = 1, kFastAO = 1 };
+  enum { kWide = 0, kHyb = 0, kGI = 1, kFastAO = 1, kTotal = 0 };
   struct State {
     Z3 z, c;
     float dr, r2;
@@ -305,7 +305,7 @@ struct Prec64 {
   typedef Prec64 Normal;
   typedef double D;
   typedef WideParams Params;
-  enum { kWide = 1, kHyb = 0, kGI = 1, kFastAO = 1 };
+  enum { kWide = 1, kHyb = 0, kGI = 1, kFastAO = 1, kTotal = 0 };
   struct State {
     double zx, zy, zz, cx, cy, cz, dr, r;
     int it, brk;  // iterations done; 1 when the loop ended by a break (bailout or NaN)
@@ -472,7 +472,7 @@ struct PrecHybT {
   static constexpr bool EXT = (FEAT & HB_EXT) != 0, ALL = (FEAT & HB_ALL) != 0;
   static constexpr bool KEEP_R = (FEAT & (HB_ALL | HB_BLEND)) != 0;  // the general kernels
   // the general kernels take GI frames of every scene and fast AO
-  enum { kWide = 0, kHyb = 1, kGI = (FEAT & HB_SEQ) != 0, kFastAO = (FEAT & HB_BLEND) != 0 };
+  enum { kWide = 0, kHyb = 1, kGI = (FEAT & HB_SEQ) != 0, kFastAO = (FEAT & HB_BLEND) != 0, kTotal = 0 };
   struct State {
     float zx, zy, zz, cx, cy, cz, dr, r;  // r: |z|, with KEEP_R only
     int it, brk;
@@ -710,7 +710,8 @@ __device__ __forceinline__ void run_stage(Stage &S, const typename P::Params &fp
       int iters;
       const typename P::D d = P::template distance<FK>(e, fp, S.detail(), iters);
       de_n++;
-      it_n += (unsigned long long)iters;
+      if constexpr (P::kTotal) it_n += (unsigned long long)e.total;  // the iterations of all orbits of the estimate
+      else it_n += (unsigned long long)iters;
       typename Stage::Real qx, qy, qz;
       if (S.step(d, iters, qx, qy, qz)) {
         P::template start<FK>(e, Stage::kMulti ? S.params() : fpk, qx, qy, qz);
