@@ -1894,7 +1894,8 @@ int pipeline_fp64(int fk, const mbr_tuning &tu, cudaStream_t st, const DevFrame 
 int pipeline_batch_fp32(int fk, const mbr_tuning &tu, cudaStream_t st, const DevFrame &fr, const FastParams &fp,
                         const WJob &j0, const Launch &L, const DevOutputs &out, long long pixels);
 int pipeline_batch_fp64(int fk, const mbr_tuning &tu, cudaStream_t st, const DevFrame &fr, const WideParams &fp,
-                        const WJob &j0, const Launch &L, const DevOutputs &out, long long pixels);
+                        const WJob &j0, const Launch &L, const DevOutputs &out, long long pixels,
+                        cudaEvent_t before_shade);
 int pipeline_hybrid(const DevScene &sc, const mbr_tuning &tu, cudaStream_t st, const DevFrame &fr, const WJob &j0,
                     const Launch &L, const DevOutputs &out, long long pixels);
 
@@ -1910,7 +1911,7 @@ static int sm_count() {
 template <bool MULTI, class P>
 static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const DevFrame &fr,
                            const typename P::Params &fp0, const WJob &j0, const Launch &L0, const DevOutputs &out,
-                           long long pixels) {
+                           long long pixels, cudaEvent_t before_shade = nullptr) {
   Launch L = L0;
   L.div_per = make_fastdiv(std::max(1, L.shadow_tasks + L.ao_rays));
   L.gate_value = P::kWide;
@@ -1989,8 +1990,13 @@ static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const 
   STAGE(primary_kernel, fr, fp0, j0, L, out)
   const bool need_normal = fr.shading_enable || L.ao_rays > 0 || L.want_normal;
   if (need_normal) { typedef typename P::Normal PN; STAGEP(PN, normal_kernel, fr, fp0, L, out) }
-  if (L.ao_rays > 0 || L.shadow_tasks > 0) {
-    direction_kernel<MULTI><<<sms * 8, 256, 0, st>>>(fr, L);
+  const bool marches = L.ao_rays > 0 || L.shadow_tasks > 0;
+  if (marches) direction_kernel<MULTI><<<sms * 8, 256, 0, st>>>(fr, L);
+  if (before_shade) {
+    e = int(cudaEventRecord(before_shade, st));
+    if (e) return e;
+  }
+  if (marches) {
     if constexpr (P::kFastAO) {
       if (L.ao_fast) { STAGE(shade_fast_kernel, fr, fp0, L, out) }
     }

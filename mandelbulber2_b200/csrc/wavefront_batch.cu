@@ -8,7 +8,7 @@ int pipeline_batch_fp32(int fk, const mbr_tuning &tu, cudaStream_t st, const Dev
 }
 
 int pipeline_batch_fp64(int fk, const mbr_tuning &tu, cudaStream_t st, const DevFrame &fr, const WideParams &fp, const WJob &j0,
-                        const Launch &L, const DevOutputs &out, long long pixels) {
-  return launch_pipeline<true, Prec64>(fk, tu, st, fr, fp, j0, L, out, pixels);
+                        const Launch &L, const DevOutputs &out, long long pixels, cudaEvent_t before_shade) {
+  return launch_pipeline<true, Prec64>(fk, tu, st, fr, fp, j0, L, out, pixels, before_shade);
 }
 }  // namespace mbr
