@@ -1,7 +1,8 @@
 """The plain FP64 engines' staged frames (csrc/staged_plain.cuh): single pixels,
 ragged sizes, row bands, the modes whose rules the stages restate, and frames
 queued on two streams of one context.  The strict engine is held to the oracle
-bit for bit, counters included."""
+bit for bit, counters included.  Frames with four AO rays go through the stages
+at every size, scenes with a primitive whatever the frame asks for."""
 import numpy as np
 import pytest
 
@@ -16,12 +17,17 @@ NAMES = ("depth", "iters", "hit", "normal", "shade", "ao", "rgb", "rgb8")
 def _case(name):
     sc = configs.mandelbox_scene(-1.5, 0.5, 30)
     p = configs.base_params(5, 20.0)
-    p.ao_rays = 3
+    p.ao_rays = 4
     p.ambient_intensity = 0.4
+    if name in ("fast_ao", "fast_ao_of_one", "steps", "unlit"):
+        sc.n_primitives = 1
+        sc.primitive[0] = abi.primitive_defaults(abi.PRIMITIVE_SPHERE)
+        sc.primitive[0].position[:] = [1.8, -1.9, 0.4]
+        sc.primitive[0].radius = 0.6
     if name == "interior":
         sc.interior_mode = 1
     elif name == "threshold":
-        sc = configs.menger_scene(6)
+        sc = configs.mandelbox_scene(-1.5, 0.5, 6)
         sc.iteration_threshold_mode = 1
     elif name == "soft":
         p.soft_shadow_cone, p.penetrating = 12.0, 1
