@@ -229,30 +229,37 @@ __device__ __forceinline__ void it_mandelbox(Z3 &z, float &dr, const Z3 &c, cons
   }
 }
 
-// (re + i im)^n for n >= 1 by binary exponentiation.
-__device__ __forceinline__ void cpow_int(float &re, float &im, int n) {
-  float ar = re, ai = im;  // the result so far (the lowest set bit of n taken first)
+// (re + i im)^n and (re2 + i im2)^n for n >= 1 by binary exponentiation: the
+// two chains share the loop and overlap their latencies (one loop each: stages
+// P / N / S of the 512x512 Mandelbulb 364 / 112 / 160 us, together 321 / 87 /
+// 147 us, the march jitter without a division included).
+__device__ __forceinline__ void cpow2_int(float &re, float &im, float &re2, float &im2, int n) {
+  // the results so far (the lowest set bit of n taken first)
   while (!(n & 1)) {
-    const float t = fmaf(ar, ar, -ai * ai);
-    ai = 2.0f * ar * ai;
-    ar = t;
+    const float t = fmaf(re, re, -im * im), t2 = fmaf(re2, re2, -im2 * im2);
+    im = 2.0f * re * im;
+    im2 = 2.0f * re2 * im2;
+    re = t;
+    re2 = t2;
     n >>= 1;
   }
-  float br = ar, bi = ai;
+  float br = re, bi = im, br2 = re2, bi2 = im2;
   n >>= 1;
   while (n) {
-    const float t = fmaf(br, br, -bi * bi);
+    const float t = fmaf(br, br, -bi * bi), t2 = fmaf(br2, br2, -bi2 * bi2);
     bi = 2.0f * br * bi;
+    bi2 = 2.0f * br2 * bi2;
     br = t;
+    br2 = t2;
     if (n & 1) {
-      const float u = fmaf(ar, br, -ai * bi);
-      ai = fmaf(ar, bi, ai * br);
-      ar = u;
+      const float u = fmaf(re, br, -im * bi), u2 = fmaf(re2, br2, -im2 * bi2);
+      im = fmaf(re, bi, im * br);
+      im2 = fmaf(re2, bi2, im2 * br2);
+      re = u;
+      re2 = u2;
     }
     n >>= 1;
   }
-  re = ar;
-  im = ai;
 }
 
 // One Mandelbulb iteration (asin latitude form of fractal_mandelbulb.cpp:32-42) + c-addition.
@@ -273,8 +280,7 @@ __device__ __forceinline__ void it_mandelbulb(Z3 &z, float &dr, const Z3 &c, con
       cp = z.x * irho;
       sp = z.y * irho;
     }
-    cpow_int(ct, st, n);
-    cpow_int(cp, sp, n);
+    cpow2_int(ct, st, cp, sp, n);
     float rn = r;  // r^n
     {
       float b = r;

@@ -21,6 +21,7 @@
 //   CalculatePixel + 8 bit    src/cimage.cpp:317-375, 460-469
 #pragma once
 #include "de_core.cuh"
+#include "jitter.h"
 
 namespace mbr {
 
@@ -244,7 +245,7 @@ __device__ MarchOut ray_marching(const DevScene &sc, const DevFrame &fr, D3 star
       found = true;
       break;
     }
-    const double jit = fr.jitter ? (1.0 - pm.random(1000) / 10000.0) : 1.0;
+    const double jit = fr.jitter ? (1.0 - tenthousandths(pm.random(1000))) : 1.0;
     if (sc.interior)
       step = (dist - 0.8 * distThresh) * fr.de_factor * jit;
     else

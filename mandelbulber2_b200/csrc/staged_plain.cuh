@@ -224,7 +224,7 @@ struct RefPrimaryStage {
       stp *= 0.5;
       return refine(qx, qy, qz);
     }
-    const double jit = fr.jitter ? (1.0 - pm.random(1000) / 10000.0) : 1.0;
+    const double jit = fr.jitter ? (1.0 - tenthousandths(pm.random(1000))) : 1.0;
     if (sc.interior)
       stp = (dist - 0.8 * thr) * fr.de_factor * jit;
     else

@@ -754,12 +754,15 @@ __device__ __forceinline__ void flush_counts(const DevOutputs &out, unsigned int
 // latency-bound: 1080p x 16 spp GI, stage GP at no bound (88 registers) / 85 /
 // 64 / 51: 87.2 / 80.4 / 76.4 / 76.8 ms; an 800x600 Mandelbox with primitives,
 // stage P at 107 / 128 / 85 / 64: 1.27 / 1.20 / 1.35 / 1.40 ms, stage S 2.46 /
-// 2.33 / 2.00 / 2.14 ms.
+// 2.33 / 2.00 / 2.14 ms.  The FP32 Mandelbox's stage P on the 1080p frame at
+// 89 / 128 / 85 / 64 registers: 1.13 / 1.30 / 1.05 / 0.99 ms (the Mandelbulb's is
+// best unbounded, 512x512: 321 / 366 / 317 / 346 us).
 template <int FK, bool MULTI, class P>
 struct kMinBlocks {
   static constexpr bool box64 = P::kWide && FK == FK_BOX_SIMPLE;
   static constexpr bool lean = P::kHyb && !P::kFastAO;  // a reference-order kernel of few formulas
-  static constexpr int primary = box64 ? (MULTI ? 3 : 4) : lean ? 2 : 0;  // 0: none asked
+  static constexpr bool box32 = !P::kWide && !P::kHyb && !MULTI && FK == FK_BOX_SIMPLE;
+  static constexpr int primary = box64 ? (MULTI ? 3 : 4) : lean ? 2 : box32 ? 4 : 0;  // 0: none asked
   static constexpr int shade = box64 ? (MULTI ? 2 : 3) : lean ? 3 : 0;
   static constexpr int gi = lean ? 4 : 0;
 };
@@ -991,7 +994,7 @@ struct PrimaryStage {
     if (fr.jitter) {
       ParkMiller p;
       p.s = pm;
-      jit = 1.0 - p.random(1000) / 10000.0;
+      jit = 1.0 - tenthousandths(p.random(1000));
       pm = p.s;
     }
     if (P::kWide) {
@@ -1681,7 +1684,7 @@ struct GIPrimaryStage {
     if (fr.jitter) {
       ParkMiller p;
       p.s = pm;
-      jit = 1.0 - p.random(1000) / 10000.0;
+      jit = 1.0 - tenthousandths(p.random(1000));
       pm = p.s;
     }
     stp = (double(d) - 0.5 * thr) * fr.de_factor * jit;
