@@ -107,21 +107,26 @@ DEFAULT_ENGINE = {"mandelbox_1080p_A": "wavefront_fp32", "mandelbox_1080p_B": "w
                   "batch_2048": "wavefront_auto"}
 
 
-def kernels_per_frame(engine: str, p) -> int:
-    """Kernel launches of one frame: the plain engines launch one kernel; the
+def kernels_per_frame(engine: str, p, formula: str, pixels: int) -> int:
+    """Kernel launches of one frame: the plain engines launch one kernel, or
+    stages P, N, S (shadow or AO) and the finish kernel for FP64 frames with 4
+    AO rays or 2^18 pixels and more (never the Menger sponge or GI); the
     wavefront pipeline launches stage P, N (normals wanted), D and S (shadow or
     AO), the finish kernel and the pixel counter; a GI frame launches the
     primary paths, per bounce level (bounces + 1 of them) the normal and vertex
     stages, the per-pixel sum and the pixel counter; the auto engine launches
     the policy kernel and both pipelines, whose kernels of the precision not
     chosen return at once."""
+    marches = p.ao_rays > 0 or (p.shading_enable and p.shadow_enable)
     if "wavefront" not in engine:
-        return 1
+        staged = ("fp64" in engine and p.gi_samples == 0 and formula != "menger"
+                  and (p.ao_rays >= 4 or pixels >= 1 << 18))
+        return (4 if marches else 3) if staged else 1
     if p.gi_samples > 0:
         n = 1 + 2 * (p.gi_bounces + 1) + 2
         return 1 + 2 * n if engine == "wavefront_auto" else n
     n = 4  # primary, normals (the bench asks for normals), finish, pixel count
-    if p.ao_rays > 0 or (p.shading_enable and p.shadow_enable):
+    if marches:
         n += 2  # directions, shadow/AO marches
     if engine == "wavefront_auto":
         return 1 + 2 * n
@@ -474,7 +479,7 @@ def run_batch(a, torch, dist, world, rank, local) -> None:
     sd = stats_dict(stats)
     fast = {k: v.cpu().numpy() for k, v in bufs.items()}
     lib.mbr_batch_destroy(b)
-    # plain FP64, job by job (one launch per job)
+    # plain FP64, job by job (one frame per job)
     base = None
     if not a.no_baseline:
         bstats = torch.zeros(len(STATS_FIELDS), dtype=torch.int64, device=r.device)
@@ -504,7 +509,7 @@ def run_batch(a, torch, dist, world, rank, local) -> None:
                 inside[offsets[i]: offsets[i] + n] = True
         out_both = both & ~inside
         rel_out = np.abs(fast["depth"][out_both] - ref["depth"][out_both]) / ref["depth"][out_both]
-        base = {"engine": "plain_fp64 (one launch per job)", "value": bsd["de_evals"] / bt, "unit": UNIT,
+        base = {"engine": "plain_fp64 (one frame per job)", "value": bsd["de_evals"] / bt, "unit": UNIT,
                 "seconds": bt, "mpix_per_s": bsd["pixels"] / bt / 1e6,
                 "hit_mismatch": float((hf != hr).mean()), "depth_rel_median": float(np.median(rel)),
                 "depth_rel_p99": float(np.quantile(rel, 0.99)),
@@ -702,7 +707,8 @@ def main() -> None:
             "de_evals_per_frame": st["de_evals"] / a.steps, "stats_per_frame": {k: v / a.steps for k, v in st.items()},
             "fp64_baseline": base, "speedup_vs_fp64": (value / base["value"]) if base else None,
             "error_vs_fp64": err, "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
-            "gpu_launches": a.steps * kernels_per_frame(a.engine, p), "clocks": clk, "per_step_ms": ms,
+            "gpu_launches": a.steps * kernels_per_frame(a.engine, p, desc["formula"], cam.width * cam.height),
+            "clocks": clk, "per_step_ms": ms,
         }
         print(json.dumps(line), flush=True)
     r.close()

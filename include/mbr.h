@@ -100,9 +100,11 @@ typedef enum mbr_de_method {
 
 /* Which kernel renders a frame. */
 typedef enum mbr_engine {
-  /* One FP64 thread per pixel; FMA contraction allowed (the plain FP64 path). */
+  /* The reference's arithmetic in FP64, one thread per pixel or, where that is
+   * faster, by stages over pixels, hits and marches; FMA contraction allowed
+   * (the plain FP64 path). */
   MBR_ENGINE_PLAIN_FP64 = 0,
-  /* Same kernel compiled without FMA contraction: every double operation is
+  /* Same kernels compiled without FMA contraction: every double operation is
    * the IEEE-rounded operation the CPU reference performs. */
   MBR_ENGINE_PLAIN_FP64_STRICT = 1,
   /* One thread per pixel; formula iteration and march step in FP32, ray
