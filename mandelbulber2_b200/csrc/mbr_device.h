@@ -209,6 +209,23 @@ __host__ __device__ inline bool scene_extended(const DevScene &sc) {
          sc.delta_de || sc.de_final > DEF_LINEAR_OFFSET || sc.n_nodes > 0;
 }
 
+// Calls f with every slot that a pass of the scene's orbit can run: the entries
+// of the sequence table (an orbit longer than the table repeats the first).  An
+// empty slot is among them where no slot is live at iteration 0: the table is
+// then one entry long and names slot 0, whatever it holds.
+template <class Fn>
+inline void for_orbit_slots(const DevScene &sc, Fn f) {
+  for (int i = 0; i < sc.length; i++) f(sc.slot[sc.seq[i]]);
+}
+
+// Whether a pass blends: a slot of the orbit has a weight other than 1 (an
+// empty slot's is 0: its pass leaves the point where it is).
+inline bool orbit_blends(const DevScene &sc) {
+  bool blend = false;
+  for_orbit_slots(sc, [&](const DevSlot &s) { blend = blend || s.d[P_WEIGHT] != 1.0; });
+  return blend;
+}
+
 // Everything about one frame that is not the scene: camera, march and
 // shading parameters, derived on the host.
 struct DevFrame {

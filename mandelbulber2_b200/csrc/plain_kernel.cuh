@@ -322,8 +322,6 @@ int launch_distance_t(const DevScene &sc, const double *pts, int64_t n, double d
   const dim3 grid(unsigned((n + 127) / 128));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool ext = scene_extended(sc);
-  bool blend = false;
-  for (int k = 0; k < sc.n; k++) blend = blend || sc.slot[k].d[P_WEIGHT] != 1.0;
   if (sc.has_w) {
     if constexpr (sizeof(T) == 8) {
       if (ext) distance_kernel<T, F_EXT, true, V><<<grid, block, 0, s>>>(sc, pts, n, detail, normal_mode, dist, iters);
@@ -333,7 +331,7 @@ int launch_distance_t(const DevScene &sc, const double *pts, int64_t n, double d
     }
   } else if (ext) {
     distance_kernel<T, F_EXT, false, V><<<grid, block, 0, s>>>(sc, pts, n, detail, normal_mode, dist, iters);
-  } else if (blend) {
+  } else if (orbit_blends(sc)) {
     distance_kernel<T, 0, false, V><<<grid, block, 0, s>>>(sc, pts, n, detail, normal_mode, dist, iters);
   } else {
     int dev = 0, sms = 148;

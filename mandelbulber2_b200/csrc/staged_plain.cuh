@@ -638,8 +638,6 @@ int launch_staged_plain_t(const DevScene &sc, const DevFrame &fr, const DevOutpu
   const RefLaunch L = ref_launch(fr, scratch);
   int e = int(cudaMemsetAsync(L.ctr, 0, sizeof(Counters4), s));
   if (e) return e;
-  bool blend = false;
-  for (int k = 0; k < sc.n; k++) blend = blend || sc.slot[k].d[P_WEIGHT] != 1.0;
   const int F = sc.is_hybrid ? 0 : sc.uniform_formula;
 #define WHOLE(FF, EXT) ref_stages<RefWhole<T, FF, false>, RefWhole<T, FF, true>, FK_ANY, EXT, V>(sc, fr, L, out, s)
 #define PASS(FF, FK) ref_stages<RefPass<T, FF, false>, RefPass<T, FF, true>, FK, false, V>(sc, fr, L, out, s)
@@ -653,7 +651,7 @@ int launch_staged_plain_t(const DevScene &sc, const DevFrame &fr, const DevOutpu
   } else if (F == MBR_FORMULA_MANDELBOX) {
     e = PASS(MBR_FORMULA_MANDELBOX, FK_BOX);
   } else {
-    e = blend ? WHOLE(0, false) : PASS(0, FK_ANY);
+    e = orbit_blends(sc) ? WHOLE(0, false) : PASS(0, FK_ANY);
   }
 #undef WHOLE
 #undef PASS

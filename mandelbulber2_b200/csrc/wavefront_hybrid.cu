@@ -14,17 +14,15 @@ int pipeline_hybrid(const DevScene &sc, const mbr_tuning &tu, cudaStream_t st, c
                     const Launch &L, const DevOutputs &out, long long pixels) {
   const HybParams hp{sc};
 #define HYBRID(FEAT) return launch_pipeline<false, PrecHybT<(FEAT)>>(FK_ANY, tu, st, fr, hp, j0, L, out, pixels)
-  bool blend = false;
+  const bool blend = orbit_blends(sc);
   int forms = 0;
-  for (int k = 0; k < sc.n; k++) {
-    const DevSlot &s = sc.slot[k];
-    if (s.formula == MBR_FORMULA_NONE) continue;  // never in the sequence
-    blend = blend || s.d[P_WEIGHT] != 1.0;
+  for_orbit_slots(sc, [&](const DevSlot &s) {  // an empty slot blends, which takes the general kernel
     forms |= s.formula == MBR_FORMULA_MANDELBULB  ? HB_BULB
              : s.formula == MBR_FORMULA_MANDELBOX ? HB_BOX
              : s.formula == MBR_FORMULA_MENGER_SPONGE ? HB_MENGER
-                                                      : HB_ALL;
-  }
+             : s.formula == MBR_FORMULA_NONE ? 0
+                                             : HB_ALL;
+  });
   if (scene_extended(sc)) {
     if (!sc.is_hybrid && !blend && fr.gi_samples == 0 && !L.ao_fast) {
       if (forms == HB_BOX) HYBRID(HB_EXT | HB_BOX);
