@@ -549,14 +549,16 @@ __global__ void __launch_bounds__(256) ref_finish_kernel(const __grid_constant__
 // than they even out (per-pixel / stages: Mandelbulb without AO 256x192 694 /
 // 752 us, 400x300 1274 / 1513, 640x480 3077 / 2671, 1024x768 7490 / 5316; with 4
 // AO rays 64x48 322 / 296, 400x300 2041 / 1871, 1024x768 14449 / 7001; Mandelbox
-// without AO 256x192 233 / 257, 640x480 1076 / 776).
+// without AO 256x192 233 / 257, 640x480 1076 / 776).  The size is the frame's,
+// whatever rows of it are asked for: a band of a frame has to equal the frame's
+// rows bit for bit, so it takes the frame's kernels.
 inline bool staged_plain_takes(const DevScene &sc, const DevFrame &fr, bool strict) {
   bool delta = sc.delta_de != 0;
   for (int k = 0; k < sc.n_nodes; k++) delta = delta || sc.node[k].delta_de != 0;
   if (sc.has_w || fr.gi_samples > 0 || fr.refine != MBR_REFINE_REFERENCE || fr.slow_shading || (delta && !strict)) return false;
   if (scene_extended(sc)) return true;
   if (!sc.is_hybrid && sc.uniform_formula == MBR_FORMULA_MENGER_SPONGE) return false;
-  return fr.ao_rays >= 4 || (long long)fr.width * (fr.row1 - fr.row0) >= 262144;
+  return fr.ao_rays >= 4 || (long long)fr.width * fr.height >= 262144;
 }
 
 // Scratch bytes of a frame.
