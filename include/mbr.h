@@ -548,7 +548,13 @@ mbr_status mbr_scene_sequence(const mbr_scene *scene, int32_t *seq_out, int32_t 
 /* Renders one frame of the current scene: the body of cRenderWorker::doWork
  * for every pixel (render_worker.cpp:126-525) on `stream`.  Asynchronous:
  * returns after the launches are queued.  Call mbr_sync to wait and to read
- * the watchdog status. */
+ * the watchdog status.
+ *
+ * A frame of the plain FP64 engines recorded into a CUDA graph takes the
+ * per-pixel kernels, which need no scratch: the graph holds kernel nodes only.
+ * On MBR_ENGINE_PLAIN_FP64 their contraction differs from that of the stages,
+ * in the last bits of a depth; MBR_ENGINE_PLAIN_FP64_STRICT gives the same bits
+ * either way. */
 mbr_status mbr_render(mbr_ctx *ctx, const mbr_camera *camera, const mbr_render_params *params,
                       const mbr_outputs *out, int engine, void *stream);
 

@@ -1053,13 +1053,18 @@ static cudaMemPool_t frame_pool_of(mbr_ctx *ctx) {
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = ctx->device;
-    if (cudaMemPoolCreate(&f.pool, &props) != cudaSuccess) {
+    // another thread may be recording in the global mode, which would refuse this
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t made = cudaMemPoolCreate(&f.pool, &props);
+    uint64_t keep = 2ull << 30;
+    if (made == cudaSuccess) cudaMemPoolSetAttribute(f.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (made != cudaSuccess) {
       cudaGetLastError();
       f.pool = nullptr;
       return nullptr;
     }
-    uint64_t keep = 2ull << 30;
-    cudaMemPoolSetAttribute(f.pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
   if (!ctx->uses_frame_pool) {
     ctx->uses_frame_pool = true;
@@ -1080,9 +1085,17 @@ void frame_pool_release(int device) {
 // Scratch of one staged plain frame, allocated and freed in the stream's
 // order: frames queued on several streams, by several threads' contexts, each
 // have their own.  Null where the frame would take more than 22 GiB (an eighth
-// of this GPU's memory) or none is left: the per-pixel kernels need none.
+// of this GPU's memory) or none is left: the per-pixel kernels need none.  Null
+// also while the stream is recorded into a caller's graph: allocation nodes
+// would keep that graph from being cloned, instantiated twice or made a child
+// of another.
 static void *frame_scratch(mbr_ctx *ctx, size_t bytes, cudaStream_t stream) {
   if (bytes > size_t(22) << 30) return nullptr;
+  cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &recording) != cudaSuccess || recording != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return nullptr;
+  }
   cudaMemPool_t pool = frame_pool_of(ctx);
   void *p = nullptr;
   if (!pool || cudaMallocFromPoolAsync(&p, bytes, pool, stream) != cudaSuccess) {
