@@ -550,11 +550,17 @@ mbr_status mbr_scene_sequence(const mbr_scene *scene, int32_t *seq_out, int32_t 
  * returns after the launches are queued.  Call mbr_sync to wait and to read
  * the watchdog status.
  *
- * A frame of the plain FP64 engines recorded into a CUDA graph takes the
- * per-pixel kernels, which need no scratch: the graph holds kernel nodes only.
- * On MBR_ENGINE_PLAIN_FP64 their contraction differs from that of the stages,
- * in the last bits of a depth; MBR_ENGINE_PLAIN_FP64_STRICT gives the same bits
- * either way. */
+ * Device memory of a frame on the plain FP64 engines: where the stages render
+ * it (see MBR_ENGINE_PLAIN_FP64), 84 bytes and 8 per AO ray for each pixel,
+ * allocated and freed in the stream's order, but at most a 64th of the device's
+ * memory: larger frames are rendered in bands of rows over that much.  Frames in
+ * flight on several streams take it each.  Between frames the contexts of a
+ * device keep at most as much together, until the last is destroyed.  The
+ * per-pixel kernels, which need none, render a frame where not even a band of
+ * four rows can be had, and one recorded into a CUDA graph, which therefore
+ * holds kernel nodes only.  On MBR_ENGINE_PLAIN_FP64 their contraction differs
+ * from that of the stages, in the last bits of a depth;
+ * MBR_ENGINE_PLAIN_FP64_STRICT gives the same bits either way. */
 mbr_status mbr_render(mbr_ctx *ctx, const mbr_camera *camera, const mbr_render_params *params,
                       const mbr_outputs *out, int engine, void *stream);
 

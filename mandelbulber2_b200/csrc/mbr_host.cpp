@@ -23,6 +23,7 @@
 #include "../../include/mbr.h"
 #include "mbr_device.h"
 #include "bailout.h"
+#include "frame_bands.h"
 #include "mbr_internal.h"
 
 using namespace mbr;
@@ -1035,16 +1036,18 @@ mbr_status ctx_work(mbr_ctx *ctx, size_t words, unsigned long long **out) {
 // The memory pool of a device's staged frames: shared by its contexts (a new
 // context's first frame finds the memory of the others' earlier frames: a
 // 801x451 frame's first pass 2.94 -> 2.31 ms), created by the first context that
-// renders such a frame and destroyed with the last one.  Between frames it
-// keeps at most 2 GiB.
+// renders such a frame and destroyed with the last one.  A frame's scratch, and
+// what the pool keeps between frames, is at most a 64th of the device's memory
+// (2.8 of 179 GiB): larger frames are rendered in bands.
 struct FramePool {
   cudaMemPool_t pool = nullptr;
+  size_t limit = 0;
   int users = 0;
 };
 static std::mutex g_frame_pool_mutex;
 static std::map<int, FramePool> &g_frame_pools = *new std::map<int, FramePool>;  // contexts may be destroyed at exit
 
-static cudaMemPool_t frame_pool_of(mbr_ctx *ctx) {
+static cudaMemPool_t frame_pool_of(mbr_ctx *ctx, size_t *limit) {
   std::lock_guard<std::mutex> lock(g_frame_pool_mutex);
   FramePool &f = g_frame_pools[ctx->device];
   if (!f.pool) {
@@ -1056,9 +1059,14 @@ static cudaMemPool_t frame_pool_of(mbr_ctx *ctx) {
     // another thread may be recording in the global mode, which would refuse this
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t made = cudaMemPoolCreate(&f.pool, &props);
-    uint64_t keep = 2ull << 30;
-    if (made == cudaSuccess) cudaMemPoolSetAttribute(f.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    size_t free_bytes = 0, total = 0;
+    cudaError_t made = cudaMemGetInfo(&free_bytes, &total);
+    if (made == cudaSuccess) made = cudaMemPoolCreate(&f.pool, &props);
+    if (made == cudaSuccess) {
+      f.limit = total / 64;
+      uint64_t keep = f.limit;
+      cudaMemPoolSetAttribute(f.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
     cudaThreadExchangeStreamCaptureMode(&mode);
     if (made != cudaSuccess) {
       cudaGetLastError();
@@ -1070,6 +1078,7 @@ static cudaMemPool_t frame_pool_of(mbr_ctx *ctx) {
     ctx->uses_frame_pool = true;
     f.users++;
   }
+  *limit = f.limit;
   return f.pool;
 }
 
@@ -1082,27 +1091,48 @@ void frame_pool_release(int device) {
   }
 }
 
-// Scratch of one staged plain frame, allocated and freed in the stream's
-// order: frames queued on several streams, by several threads' contexts, each
-// have their own.  Null where the frame would take more than 22 GiB (an eighth
-// of this GPU's memory) or none is left: the per-pixel kernels need none.  Null
-// also while the stream is recorded into a caller's graph: allocation nodes
-// would keep that graph from being cloned, instantiated twice or made a child
-// of another.
-static void *frame_scratch(mbr_ctx *ctx, size_t bytes, cudaStream_t stream) {
-  if (bytes > size_t(22) << 30) return nullptr;
+// One plain FP64 frame by stages; false where the per-pixel kernels, which need
+// no scratch, have to render it: frames that the stages do not take, a stream
+// that is recorded into a caller's graph (allocation nodes would keep that graph
+// from being cloned, instantiated twice or made a child of another), or no
+// memory for the smallest band.  The scratch is allocated and freed in the
+// stream's order: frames queued on several streams, by several threads'
+// contexts, each have their own.
+static bool render_staged(mbr_ctx *ctx, const DevScene &sc, const DevFrame &fr, const DevOutputs &out, bool strict,
+                          cudaStream_t stream, int *err) {
+  if (!staged_plain_scratch(sc, fr, strict)) return false;
   cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &recording) != cudaSuccess || recording != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
-    return nullptr;
+    return false;
   }
-  cudaMemPool_t pool = frame_pool_of(ctx);
-  void *p = nullptr;
-  if (!pool || cudaMallocFromPoolAsync(&p, bytes, pool, stream) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
+  size_t limit = 0;
+  const cudaMemPool_t pool = frame_pool_of(ctx, &limit);
+  if (!pool) return false;
+  DevFrame band = fr;
+  const FrameBands b = frame_bands(
+      fr.row1 - fr.row0, limit,
+      [&](int rows) {
+        band.row1 = fr.row0 + rows;
+        return staged_plain_scratch(sc, band, strict);
+      },
+      [&](size_t bytes) {
+        void *p = nullptr;
+        if (cudaMallocFromPoolAsync(&p, bytes, pool, stream) == cudaSuccess) return p;
+        cudaGetLastError();
+        return static_cast<void *>(nullptr);
+      });
+  if (!b.scratch) return false;
+  int e = 0;
+  for (int row = fr.row0; row < fr.row1 && !e; row += b.rows) {
+    band.row0 = row;
+    band.row1 = std::min(row + b.rows, fr.row1);
+    e = strict ? launch_staged_fp64_strict(sc, band, out, b.scratch, stream)
+               : launch_staged_fp64(sc, band, out, b.scratch, stream);
   }
-  return p;
+  const int f = int(cudaFreeAsync(b.scratch, stream));
+  *err = e ? e : f;
+  return true;
 }
 
 mbr_status ctx_adjoint_partials(mbr_ctx *ctx, size_t bytes, double **out) {
@@ -1386,16 +1416,9 @@ mbr_status mbr_render(mbr_ctx *ctx, const mbr_camera *camera, const mbr_render_p
   }
   int e;
   const bool strict = engine == MBR_ENGINE_PLAIN_FP64_STRICT;
-  if (strict || engine == MBR_ENGINE_PLAIN_FP64) {
-    const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const size_t need = staged_plain_scratch(*scp, fr, strict);
-    if (void *scratch = need ? frame_scratch(ctx, need, s) : nullptr) {
-      e = strict ? launch_staged_fp64_strict(*scp, fr, d, scratch, stream)
-                 : launch_staged_fp64(*scp, fr, d, scratch, stream);
-      const int f = int(cudaFreeAsync(scratch, s));
-      return cuda_err(ctx, e ? e : f, "kernel launch");
-    }
-  }
+  if ((strict || engine == MBR_ENGINE_PLAIN_FP64) &&
+      render_staged(ctx, *scp, fr, d, strict, static_cast<cudaStream_t>(stream), &e))
+    return cuda_err(ctx, e, "kernel launch");
   switch (engine) {
     case MBR_ENGINE_PLAIN_FP64: e = launch_plain_fp64(*scp, fr, d, stream); break;
     case MBR_ENGINE_PLAIN_FP64_STRICT: e = launch_plain_fp64_strict(*scp, fr, d, stream); break;
