@@ -251,6 +251,20 @@ struct mbr_batch {
 // Scratch of one group, a multiple of 256 bytes.
 static size_t group_scratch(const BatchGroup &g, int per) { return (scratch_bytes(g.items, per) + 255) / 256 * 256; }
 
+// Whether two jobs write a pixel in common.  Groups that run in turn then leave
+// the last one's; side by side they would race.
+static bool jobs_overlap(const std::vector<WJob> &jobs) {
+  std::vector<std::pair<long long, long long>> span;
+  for (const WJob &j : jobs) {
+    const long long first = j.pixel_offset + (long long)j.row0 * j.width;
+    span.push_back({first, first + (long long)j.rows * j.width});
+  }
+  std::sort(span.begin(), span.end());
+  for (size_t i = 1; i < span.size(); i++)
+    if (span[i].first < span[i - 1].second) return true;
+  return false;
+}
+
 // Precision flag of every job (AUTO): the policy kernel over the job table.
 static int batch_policy(const std::vector<DevScene> &dsc, const std::vector<int> &scene_of,
                         const std::vector<WJob> &wj, const DevFrame &fr0, std::vector<int> *flags) {
@@ -374,10 +388,11 @@ mbr_status mbr_batch_create(mbr_ctx *ctx, const mbr_scene *scenes, int32_t n_sce
   if (e) return fail(e, "cudaMalloc(wide params)");
   const int per = ((fr0.shading_enable && fr0.shadow_enable) ? 1 : 0) + ao_tasks(fr0);
   // Scratch: one region that the groups use in turn, or, where all of them fit
-  // in 16 GiB, one region each, so that the groups run side by side.
+  // in 16 GiB and no two jobs write the same pixel, one region each, so that the
+  // groups run side by side.
   size_t each = 0;
   for (const BatchGroup &g : b->groups) each += group_scratch(g, per);
-  bool side_by_side = b->groups.size() > 1 && each <= size_t(16) << 30;
+  bool side_by_side = b->groups.size() > 1 && each <= size_t(16) << 30 && !jobs_overlap(wj);
   if (side_by_side && cudaMalloc(&b->d_scratch, each) != cudaSuccess) {
     cudaGetLastError();
     b->d_scratch = nullptr;
@@ -419,6 +434,7 @@ mbr_status mbr_batch_create(mbr_ctx *ctx, const mbr_scene *scenes, int32_t n_sce
     for (int wide = 1; wide >= 0; wide--)
       for (size_t i = 0; i < b->groups.size(); i++)
         if (b->groups[i].wide == wide) order.push_back(i);
+    if (!side_by_side) std::sort(order.begin(), order.end());  // in turn: FP32 first, as the groups lie
     for (size_t i : order) {
       if (le) break;
       const BatchGroup &g = b->groups[i];
