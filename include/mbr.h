@@ -590,7 +590,13 @@ typedef struct mbr_job {
  * over its jobs with one persistent launch per stage.  Outputs are indexed
  * pixel_offset + y*width + x.  engine must be a WAVEFRONT engine; with
  * MBR_ENGINE_WAVEFRONT_AUTO the precision is chosen per job here (a
- * synchronous device evaluation of DE at every camera). */
+ * synchronous device evaluation of DE at every camera).
+ *
+ * Device memory, held until mbr_batch_destroy: per pipeline the scratch of its
+ * pixels (mbr_wavefront_scratch_layout), for all pipelines where that is at most
+ * an eighth of the device's free memory, so that they run side by side; else,
+ * and where jobs write pixels in common, the largest pipeline's, and they run in
+ * turn, the FP32 ones by formula kind, then the FP64 ones. */
 mbr_status mbr_batch_create(mbr_ctx *ctx, const mbr_scene *scenes, int32_t n_scenes,
                             const mbr_job *jobs, int32_t n_jobs,
                             const mbr_render_params *params, const mbr_outputs *out,

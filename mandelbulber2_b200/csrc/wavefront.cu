@@ -387,12 +387,15 @@ mbr_status mbr_batch_create(mbr_ctx *ctx, const mbr_scene *scenes, int32_t n_sce
   e = int(cudaMalloc(&b->d_wide, sizeof(WideParams) * n_jobs));
   if (e) return fail(e, "cudaMalloc(wide params)");
   const int per = ((fr0.shading_enable && fr0.shadow_enable) ? 1 : 0) + ao_tasks(fr0);
-  // Scratch: one region that the groups use in turn, or, where all of them fit
-  // in 16 GiB and no two jobs write the same pixel, one region each, so that the
-  // groups run side by side.
+  // Scratch: one region that the groups use in turn, or, where together they
+  // take at most an eighth of the device's free memory and no two jobs write the
+  // same pixel, one region each, so that the groups run side by side.
   size_t each = 0;
   for (const BatchGroup &g : b->groups) each += group_scratch(g, per);
-  bool side_by_side = b->groups.size() > 1 && each <= size_t(16) << 30 && !jobs_overlap(wj);
+  size_t free_bytes = 0, total_bytes = 0;
+  e = int(cudaMemGetInfo(&free_bytes, &total_bytes));
+  if (e) return fail(e, "cudaMemGetInfo");
+  bool side_by_side = b->groups.size() > 1 && each <= free_bytes / 8 && !jobs_overlap(wj);
   if (side_by_side && cudaMalloc(&b->d_scratch, each) != cudaSuccess) {
     cudaGetLastError();
     b->d_scratch = nullptr;
