@@ -754,15 +754,20 @@ __device__ __forceinline__ void flush_counts(const DevOutputs &out, unsigned int
 // latency-bound: 1080p x 16 spp GI, stage GP at no bound (88 registers) / 85 /
 // 64 / 51: 87.2 / 80.4 / 76.4 / 76.8 ms; an 800x600 Mandelbox with primitives,
 // stage P at 107 / 128 / 85 / 64: 1.27 / 1.20 / 1.35 / 1.40 ms, stage S 2.46 /
-// 2.33 / 2.00 / 2.14 ms.  The FP32 Mandelbox's stage P on the 1080p frame at
-// 89 / 128 / 85 / 64 registers: 1.13 / 1.30 / 1.05 / 0.99 ms (the Mandelbulb's is
-// best unbounded, 512x512: 321 / 366 / 317 / 346 us).
+// 2.33 / 2.00 / 2.14 ms.  The FP32 Mandelbox's stage P, from kFewPixels pixels:
+// frames without AO over six views and scales from -2 to 3, time at no bound (89
+// registers) over that at 85 / 64 / 51: 1920x1080 1.00 to 1.05 / 0.98 to 1.08 /
+// 0.94 to 1.06, 1280x720 1.00 to 1.06 / 0.95 to 1.10 / 0.82 to 1.08, 640x360 0.99
+// to 1.02 / 0.94 to 1.03 / 0.89 to 1.03.  64 registers are best on the view that
+// fills the frame with short orbits and cost where orbits are long; 85 cost 1 %
+// at most.  Below, no bound: 320x180 0.98 to 0.99 / 0.91 to 0.95 / 0.89 to 0.94
+// (the Mandelbulb's is best unbounded, 512x512: 321 / 366 / 317 / 346 us).
 template <int FK, bool MULTI, class P>
 struct kMinBlocks {
   static constexpr bool box64 = P::kWide && FK == FK_BOX_SIMPLE;
   static constexpr bool lean = P::kHyb && !P::kFastAO;  // a reference-order kernel of few formulas
   static constexpr bool box32 = !P::kWide && !P::kHyb && !MULTI && FK == FK_BOX_SIMPLE;
-  static constexpr int primary = box64 ? (MULTI ? 3 : 4) : lean ? 2 : box32 ? 4 : 0;  // 0: none asked
+  static constexpr int primary = box64 ? (MULTI ? 3 : 4) : lean ? 2 : box32 ? 3 : 0;  // 0: none asked
   static constexpr int shade = box64 ? (MULTI ? 2 : 3) : lean ? 3 : 0;
   static constexpr int gi = lean ? 4 : 0;
 };
@@ -1019,8 +1024,8 @@ struct PrimaryStage {
   }
 };
 
-template <int FK, bool MULTI, class P>
-__global__ void __launch_bounds__(256, kMinBlocks<FK, MULTI, P>::primary) primary_kernel(const __grid_constant__ DevFrame fr,
+template <int FK, bool MULTI, class P, int BLOCKS = kMinBlocks<FK, MULTI, P>::primary>
+__global__ void __launch_bounds__(256, BLOCKS) primary_kernel(const __grid_constant__ DevFrame fr,
                                                       const __grid_constant__ typename P::Params fp0,
                                                       const __grid_constant__ WJob job0,
                                                       const __grid_constant__ Launch L, DevOutputs out) {
@@ -1910,6 +1915,9 @@ static int sm_count() {
   return sms;
 }
 
+// Below this many pixels the FP32 Mandelbox's stage P runs unbounded (see kMinBlocks).
+const long long kFewPixels = 131072;
+
 // The stage launches of one frame or batch under policy P, in stream order.
 template <bool MULTI, class P>
 static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const DevFrame &fr,
@@ -1990,7 +1998,12 @@ static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const 
     STAGE_LAUNCH(PP, KERNEL, FK_ANY, __VA_ARGS__)                                       \
     default: return int(cudaErrorInvalidValue);                                         \
   }
-  STAGE(primary_kernel, fr, fp0, j0, L, out)
+  bool few = false;
+  if constexpr (kMinBlocks<FK_BOX_SIMPLE, MULTI, P>::box32) {
+    few = fk == FK_BOX_SIMPLE && L.total < kFewPixels;
+    if (few) primary_kernel<FK_BOX_SIMPLE, MULTI, P, 0><<<grid, block, 0, st>>>(fr, fp0, j0, L, out);
+  }
+  if (!few) { STAGE(primary_kernel, fr, fp0, j0, L, out) }
   const bool need_normal = fr.shading_enable || L.ao_rays > 0 || L.want_normal;
   if (need_normal) { typedef typename P::Normal PN; STAGEP(PN, normal_kernel, fr, fp0, L, out) }
   const bool marches = L.ao_rays > 0 || L.shadow_tasks > 0;
