@@ -316,7 +316,7 @@ int launch_plain_fp64(const DevScene &sc, const DevFrame &fr, const DevOutputs &
 int launch_plain_fp64_strict(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *stream);
 // The same frames by stages (staged_plain.cuh): the scratch bytes a frame
 // needs, 0 where the per-pixel kernels render it, and the launch.
-size_t staged_plain_scratch(const DevScene &sc, const DevFrame &fr, bool strict);
+size_t staged_plain_scratch(const DevScene &sc, const DevFrame &fr);
 int launch_staged_fp64(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *scratch, void *stream);
 int launch_staged_fp64_strict(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *scratch, void *stream);
 int launch_plain_mixed(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *stream);

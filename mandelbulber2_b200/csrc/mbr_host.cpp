@@ -1100,7 +1100,7 @@ void frame_pool_release(int device) {
 // contexts, each have their own.
 static bool render_staged(mbr_ctx *ctx, const DevScene &sc, const DevFrame &fr, const DevOutputs &out, bool strict,
                           cudaStream_t stream, int *err) {
-  if (!staged_plain_scratch(sc, fr, strict)) return false;
+  if (!staged_plain_scratch(sc, fr)) return false;
   cudaStreamCaptureStatus recording = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &recording) != cudaSuccess || recording != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
@@ -1114,7 +1114,7 @@ static bool render_staged(mbr_ctx *ctx, const DevScene &sc, const DevFrame &fr, 
       fr.row1 - fr.row0, limit,
       [&](int rows) {
         band.row1 = fr.row0 + rows;
-        return staged_plain_scratch(sc, band, strict);
+        return staged_plain_scratch(sc, band);
       },
       [&](size_t bytes) {
         void *p = nullptr;

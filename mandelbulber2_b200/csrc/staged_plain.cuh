@@ -540,25 +540,45 @@ __global__ void __launch_bounds__(256) ref_finish_kernel(const __grid_constant__
 }
 
 // Frames the stages take: a 3-D state, the reference's refinement, no GI and
-// no iteration-count normals.  With contraction the stages round a point's last
-// bit otherwise than plain_kernel (depths within 1e-15); the delta DE magnifies
-// that 1e7-fold, so its scenes stay there.  Of the rest plain_kernel keeps what
-// it renders faster: the Menger sponge, whose estimates are short and alike
-// (64x48 to 1024x768 frames run at 0.70 to 0.95 of its speed by stages), and
-// small frames without many marches, where the stages' separate tails cost more
-// than they even out (per-pixel / stages: Mandelbulb without AO 256x192 694 /
-// 752 us, 400x300 1274 / 1513, 640x480 3077 / 2671, 1024x768 7490 / 5316; with 4
-// AO rays 64x48 322 / 296, 400x300 2041 / 1871, 1024x768 14449 / 7001; Mandelbox
-// without AO 256x192 233 / 257, 640x480 1076 / 776).  The size is the frame's,
-// whatever rows of it are asked for: a band of a frame has to equal the frame's
-// rows bit for bit, so it takes the frame's kernels.
-inline bool staged_plain_takes(const DevScene &sc, const DevFrame &fr, bool strict) {
+// no iteration-count normals.  Of these plain_kernel keeps what it renders
+// faster (per-pixel / stages, us):
+//  - The delta DE, four orbits an estimate that run alike in neighbouring pixels
+//    (strict engine: Mandelbox 160x120 7660 / 8811, 320x240 with 4 AO rays 19202 /
+//    22364; box fold bulb pow 2 320x240 6453 / 8718, with 4 rays 12628 / 10970).
+//    With contraction it would magnify the difference between the two forms'
+//    rounding (depths within 1e-15) 1e7-fold.
+//  - Explicit objects trees with fewer than 4 AO rays: a tree's walk branches by
+//    where a point lies, and neighbouring pixels, which a warp of plain_kernel
+//    marches together, branch alike.  Six trees, 64x48 to 1024x768: without AO
+//    1029 / 1188 to 12132 / 16940 (0.68 to 1.04 of its speed), 2 rays 0.83 to
+//    1.27, 4 rays 0.96 to 1.64, 8 rays 1.07 to 2.74.
+//  - Of the other extended scenes (primitives, limits, folds, rotations, other
+//    formulas and nine by settings key, 16x12 to 640x480, 0 and 4 rays: 1.04 to
+//    6.3), frames below 160x120 with fewer than 4 AO rays where the estimates are
+//    short: the Menger sponge (with a sphere 16x12 194 / 208, 128x96 519 / 548,
+//    160x120 636 / 593), the Mandelbulb (with folds 16x12 254 / 269, 64x48 649 /
+//    664, 160x120 1205 / 1077) and sequences (in a limit box 16x12 157 / 165,
+//    64x48 208 / 252, 160x120 917 / 816; with a sphere 16x12 268 / 278).
+//  - The Menger sponge without extensions (64x48 to 1024x768 frames run at 0.70 to
+//    0.95 of its speed by stages).
+//  - Small frames without many marches, where the stages' separate tails cost
+//    more than they even out: Mandelbulb without AO 256x192 694 / 752, 400x300
+//    1274 / 1513, 640x480 3077 / 2671, 1024x768 7490 / 5316; with 4 AO rays 64x48
+//    322 / 296, 400x300 2041 / 1871, 1024x768 14449 / 7001; Mandelbox without AO
+//    256x192 233 / 257, 640x480 1076 / 776.
+// The size is the frame's, whatever rows of it are asked for: a band of a frame
+// has to equal the frame's rows bit for bit, so it takes the frame's kernels.
+inline bool staged_plain_takes(const DevScene &sc, const DevFrame &fr) {
   bool delta = sc.delta_de != 0;
   for (int k = 0; k < sc.n_nodes; k++) delta = delta || sc.node[k].delta_de != 0;
-  if (sc.has_w || fr.gi_samples > 0 || fr.refine != MBR_REFINE_REFERENCE || fr.slow_shading || (delta && !strict)) return false;
-  if (scene_extended(sc)) return true;
-  if (!sc.is_hybrid && sc.uniform_formula == MBR_FORMULA_MENGER_SPONGE) return false;
-  return fr.ao_rays >= 4 || (long long)fr.width * fr.height >= 262144;
+  if (sc.has_w || fr.gi_samples > 0 || fr.refine != MBR_REFINE_REFERENCE || fr.slow_shading || delta) return false;
+  if (fr.ao_rays >= 4) return scene_extended(sc) || sc.is_hybrid || sc.uniform_formula != MBR_FORMULA_MENGER_SPONGE;
+  const long long pixels = (long long)fr.width * fr.height;
+  if (sc.n_nodes > 0) return false;
+  if (scene_extended(sc))
+    return pixels >= 19200 || !(sc.is_hybrid || sc.uniform_formula == MBR_FORMULA_MENGER_SPONGE ||
+                                sc.uniform_formula == MBR_FORMULA_MANDELBULB);
+  return pixels >= 262144 && (sc.is_hybrid || sc.uniform_formula != MBR_FORMULA_MENGER_SPONGE);
 }
 
 // Scratch bytes of a frame.
