@@ -1281,10 +1281,48 @@ __device__ __forceinline__ void keyed_formula(V4<T> &z, T r, T &DE, const DevSlo
   else if constexpr (FORMULA == MBR_FORMULA_DIFS_HEXTGRID2) f_difs_hextgrid2<T>(z, DE, ax, s, i);
   else if constexpr (FORMULA == MBR_FORMULA_MENGER_MOD1) f_menger_mod1<T>(z, DE, s, i);
 }
-// The same as a called function, for the kernels that carry every formula.
-template <class T, int FORMULA>
-__device__ __noinline__ void keyed_call(V4<T> &z, T r, T &DE, const DevSlot &s, int i, const V4<T> &c, AuxX<T> &ax) {
-  keyed_formula<T, FORMULA>(z, r, DE, s, i, c, ax);
+// The same as called functions, for the kernels that carry every formula; each
+// takes only the state its formula reads, since what is passed by reference has
+// to be in local memory around the call.
+template <class T>
+__device__ __noinline__ void call_pseudo_kleinian(V4<T> &z, T &DE, T &pk, const DevSlot &s, int i) {
+  f_pseudo_kleinian<T>(z, DE, pk, s, i);
+}
+template <class T>
+__device__ __noinline__ void call_box_fold_bulb_pow2_v2(V4<T> &z, T &DE, T &scaleA, const DevSlot &s, int i) {
+  f_box_fold_bulb_pow2_v2<T>(z, DE, scaleA, s, i);
+}
+template <class T>
+__device__ __noinline__ void call_abox_mod11(V4<T> &z, T &DE, AuxX<T> &ax, const V4<T> &c, const DevSlot &s, int i) {
+  f_abox_mod11<T>(z, DE, ax, c, s, i);
+}
+template <class T>
+__device__ __noinline__ void call_pseudo_kleinian_mod4(V4<T> &z, T &DE, AuxX<T> &ax, const DevSlot &s, int i) {
+  f_pseudo_kleinian_mod4<T>(z, DE, ax, s, i);
+}
+template <class T>
+__device__ __noinline__ void call_pseudo_kleinian_std_de(V4<T> &z, T &DE, AuxX<T> &ax, const DevSlot &s, int i) {
+  f_pseudo_kleinian_std_de<T>(z, DE, ax, s, i);
+}
+template <class T>
+__device__ __noinline__ void call_generalized_fold_box(V4<T> &z, T &DE, const DevSlot &s) {
+  f_generalized_fold_box<T>(z, DE, s);
+}
+template <class T>
+__device__ __noinline__ void call_mandelbulb_pupuku(V4<T> &z, T r, T &DE, T &dist, const DevSlot &s, int i) {
+  f_mandelbulb_pupuku<T>(z, r, DE, dist, s, i);
+}
+template <class T>
+__device__ __noinline__ void call_difs_hextgrid2(V4<T> &z, T &DE, AuxX<T> &ax, const DevSlot &s, int i) {
+  f_difs_hextgrid2<T>(z, DE, ax, s, i);
+}
+template <class T>
+__device__ __noinline__ void call_box_fold_bulb_pow2(V4<T> &z, T r, T &DE, const DevSlot &s) {
+  f_box_fold_bulb_pow2<T>(z, r, DE, s);
+}
+template <class T>
+__device__ __noinline__ void call_menger_mod1(V4<T> &z, T &DE, const DevSlot &s, int i) {
+  f_menger_mod1<T>(z, DE, s, i);
 }
 
 // EXT: the formulas beyond the three specialised ones and the Mandelbox
@@ -1298,16 +1336,16 @@ __device__ __forceinline__ void formula_dispatch(int formula, V4<T> &z, T r, T &
                                                  AuxX<T> &ax) {
   if constexpr (EXT) {
     switch (formula) {
-      case MBR_FORMULA_PSEUDO_KLEINIAN: keyed_call<T, MBR_FORMULA_PSEUDO_KLEINIAN>(z, r, DE, s, i, c, ax); break;
-      case MBR_FORMULA_BOX_FOLD_BULB_POW2_V2: keyed_call<T, MBR_FORMULA_BOX_FOLD_BULB_POW2_V2>(z, r, DE, s, i, c, ax); break;
-      case MBR_FORMULA_ABOX_MOD11: keyed_call<T, MBR_FORMULA_ABOX_MOD11>(z, r, DE, s, i, c, ax); break;
-      case MBR_FORMULA_PSEUDO_KLEINIAN_MOD4: keyed_call<T, MBR_FORMULA_PSEUDO_KLEINIAN_MOD4>(z, r, DE, s, i, c, ax); break;
-      case MBR_FORMULA_PSEUDO_KLEINIAN_STD_DE: keyed_call<T, MBR_FORMULA_PSEUDO_KLEINIAN_STD_DE>(z, r, DE, s, i, c, ax); break;
-      case MBR_FORMULA_GENERALIZED_FOLD_BOX: keyed_call<T, MBR_FORMULA_GENERALIZED_FOLD_BOX>(z, r, DE, s, i, c, ax); break;
-      case MBR_FORMULA_MANDELBULB_PUPUKU: keyed_call<T, MBR_FORMULA_MANDELBULB_PUPUKU>(z, r, DE, s, i, c, ax); break;
-      case MBR_FORMULA_DIFS_HEXTGRID2: keyed_call<T, MBR_FORMULA_DIFS_HEXTGRID2>(z, r, DE, s, i, c, ax); break;
-      case MBR_FORMULA_BOX_FOLD_BULB_POW2: keyed_call<T, MBR_FORMULA_BOX_FOLD_BULB_POW2>(z, r, DE, s, i, c, ax); break;
-      case MBR_FORMULA_MENGER_MOD1: keyed_call<T, MBR_FORMULA_MENGER_MOD1>(z, r, DE, s, i, c, ax); break;
+      case MBR_FORMULA_PSEUDO_KLEINIAN: call_pseudo_kleinian<T>(z, DE, ax.pk, s, i); break;
+      case MBR_FORMULA_BOX_FOLD_BULB_POW2_V2: call_box_fold_bulb_pow2_v2<T>(z, DE, ax.scaleA, s, i); break;
+      case MBR_FORMULA_ABOX_MOD11: call_abox_mod11<T>(z, DE, ax, c, s, i); break;
+      case MBR_FORMULA_PSEUDO_KLEINIAN_MOD4: call_pseudo_kleinian_mod4<T>(z, DE, ax, s, i); break;
+      case MBR_FORMULA_PSEUDO_KLEINIAN_STD_DE: call_pseudo_kleinian_std_de<T>(z, DE, ax, s, i); break;
+      case MBR_FORMULA_GENERALIZED_FOLD_BOX: call_generalized_fold_box<T>(z, DE, s); break;
+      case MBR_FORMULA_MANDELBULB_PUPUKU: call_mandelbulb_pupuku<T>(z, r, DE, ax.dist, s, i); break;
+      case MBR_FORMULA_DIFS_HEXTGRID2: call_difs_hextgrid2<T>(z, DE, ax, s, i); break;
+      case MBR_FORMULA_BOX_FOLD_BULB_POW2: call_box_fold_bulb_pow2<T>(z, r, DE, s); break;
+      case MBR_FORMULA_MENGER_MOD1: call_menger_mod1<T>(z, DE, s, i); break;
       case MBR_FORMULA_QUATERNION: f_quaternion<T>(z, r, DE); break;
       case MBR_FORMULA_AEXION: f_aexion<T>(z, r, DE, s, i, c); break;
       case MBR_FORMULA_MANDELBULB: f_mandelbulb<T>(z, r, DE, s); break;
