@@ -266,16 +266,15 @@ struct AdjointFrame {
   double dM[9];  // d(mRot)/d(yaw)
 };
 
-// One thread per pixel: the Mandelbox (its three point and two parameter
-// tangents; with the Mandelbulb's too, at 255 registers, a 256x256 image took
-// 302 us instead of 218).
-template <class T>
+// One thread per pixel, with the formula's tangents only (with both formulas'
+// six, at 255 registers, a 256x256 Mandelbox image took 302 us instead of 218).
+template <class T, bool BULB>
 __global__ void __launch_bounds__(128) adjoint_pixel_kernel(const __grid_constant__ DevScene sc,
                                                       const __grid_constant__ DevFrame fr,
                                                       const __grid_constant__ AdjointFrame af, const double *depth,
                                                       const uint8_t *hit, const float *dl_ddepth,
                                                       const float *dl_dshade, double *partials) {
-  typedef Dn<T, Tangents<false>::n> Dual;
+  typedef Dn<T, Tangents<BULB>::n> Dual;
   const long long n = (long long)fr.width * fr.height;
   double acc[MBR_GRAD_COUNT];
 #pragma unroll
@@ -298,7 +297,7 @@ __global__ void __launch_bounds__(128) adjoint_pixel_kernel(const __grid_constan
     const double thr = dist_thresh(sc, fr, p);
     const double c0 = fr.resolution * fr.fov / fr.detail_level * d3len(dir);
     // dist and its tangents at the hit point
-    const Dual dh = de_dual<T, false>(sc, T(p.x), T(p.y), T(p.z), T(thr));
+    const Dual dh = de_dual<T, BULB>(sc, T(p.x), T(p.y), T(p.z), T(thr));
     // implicit differentiation needs F(t) = dist - thr = 0 at the stored
     // depth; a refinement that ended on a jump of the distance estimate (an
     // orbit's bailout iteration changing along the ray) has no derivative
@@ -320,8 +319,12 @@ __global__ void __launch_bounds__(128) adjoint_pixel_kernel(const __grid_constan
     double dd[MBR_GRAD_COUNT];
 #pragma unroll
     for (int k = 0; k < MBR_GRAD_COUNT; k++) dd[k] = 0.0;
-    dd[MBR_GRAD_MANDELBOX_SCALE] = double(dh.d[TN_P0]);
-    dd[MBR_GRAD_MANDELBOX_MIN_R2] = double(dh.d[TN_P1]);
+    if (BULB) {
+      dd[MBR_GRAD_BULB_POWER] = double(dh.d[TN_P0]);
+    } else {
+      dd[MBR_GRAD_MANDELBOX_SCALE] = double(dh.d[TN_P0]);
+      dd[MBR_GRAD_MANDELBOX_MIN_R2] = double(dh.d[Tangents<BULB>::n - 1]);
+    }
     const double denom = d3dot(g, dir) - c0;
     double dt[MBR_GRAD_COUNT];
 #pragma unroll
@@ -337,8 +340,8 @@ __global__ void __launch_bounds__(128) adjoint_pixel_kernel(const __grid_constan
       for (int a = 0; a < 3; a++) {
         const D3 e{a == 0 ? 1.0 : 0.0, a == 1 ? 1.0 : 0.0, a == 2 ? 1.0 : 0.0};
         const D3 pp = d3add(p, d3mul(e, delta)), pm = d3sub(p, d3mul(e, delta));
-        const Dual sp = de_dual<T, false>(sc, T(pp.x), T(pp.y), T(pp.z), T(thr));
-        const Dual sm = de_dual<T, false>(sc, T(pm.x), T(pm.y), T(pm.z), T(thr));
+        const Dual sp = de_dual<T, BULB>(sc, T(pp.x), T(pp.y), T(pp.z), T(thr));
+        const Dual sm = de_dual<T, BULB>(sc, T(pm.x), T(pm.y), T(pm.z), T(thr));
         gv[a] = double(sp.v) - double(sm.v);
         const D3 gp{double(sp.d[TN_X]), double(sp.d[TN_Y]), double(sp.d[TN_Z])};
         const D3 gm{double(sm.d[TN_X]), double(sm.d[TN_Y]), double(sm.d[TN_Z])};
@@ -348,9 +351,12 @@ __global__ void __launch_bounds__(128) adjoint_pixel_kernel(const __grid_constan
           const double ddelta = c0 * fr.smoothness * dt[k];
           double dplus = d3dot(gp, d3add(dpt, d3mul(e, ddelta)));
           double dminus = d3dot(gm, d3sub(dpt, d3mul(e, ddelta)));
-          if (k == MBR_GRAD_MANDELBOX_SCALE || k == MBR_GRAD_MANDELBOX_MIN_R2) {
-            dplus += double(sp.d[TN_P0 + k - MBR_GRAD_MANDELBOX_SCALE]);
-            dminus += double(sm.d[TN_P0 + k - MBR_GRAD_MANDELBOX_SCALE]);
+          if (k == (BULB ? MBR_GRAD_BULB_POWER : MBR_GRAD_MANDELBOX_SCALE)) {
+            dplus += double(sp.d[TN_P0]);
+            dminus += double(sm.d[TN_P0]);
+          } else if (!BULB && k == MBR_GRAD_MANDELBOX_MIN_R2) {
+            dplus += double(sp.d[Tangents<BULB>::n - 1]);
+            dminus += double(sm.d[Tangents<BULB>::n - 1]);
           }
           gd[a][k] = dplus - dminus;
         }
@@ -584,14 +590,18 @@ extern "C" mbr_status mbr_adjoint(mbr_ctx *ctx, const mbr_camera *camera, const 
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const long long n = (long long)fr.width * fr.height;
-  // Eight lanes per hit, or one thread per pixel for a Mandelbox image of 128^2
-  // pixels and more: its estimate, 12 passes without library functions, is
+  // Eight lanes per hit, or one thread per pixel: for a Mandelbox image of 128^2
+  // pixels and more, whose estimate, 12 passes without library functions, is
   // short enough that many pixels in flight hide it, and the groups' exchange
   // costs more than their parallel samples save (per pixel / eight lanes: 100x95
   // 85 / 61 us, 160x160 108 / 139 us, 256x256 218 / 319 us, 512x505 765 / 1202
-  // us; the Mandelbulb 64x60 60 / 14 us, 256x256 182 / 81 us, 512x505 1664 / 802 us).
+  // us; the Mandelbulb 64x60 60 / 14 us, 256x256 182 / 81 us, 512x505 1664 / 802
+  // us); and without a shade gradient, where a hit has one estimate and seven
+  // lanes of the group would idle (the whole call, per pixel / eight lanes:
+  // Mandelbulb 64x64 51 / 50 us, 160x160 53 / 75 us, 256x256 65 / 109 us, 400x400
+  // 89 / 202 us; Mandelbox 100x100 53 / 67 us).
   const bool bulb = sc->slot[0].formula == MBR_FORMULA_MANDELBULB;
-  const bool per_pixel = !bulb && n >= 16384;
+  const bool per_pixel = !dl_dshade || (!bulb && n >= 16384);
   const long long blocks = per_pixel ? (n + 127) / 128 : (n + 15) / 16;
   const int grid = int(std::max<long long>(1, std::min<long long>(blocks, (long long)sms * 16)));
   double *partials = nullptr;
@@ -599,12 +609,14 @@ extern "C" mbr_status mbr_adjoint(mbr_ctx *ctx, const mbr_camera *camera, const 
   if (st != MBR_OK) return st;
 #define ADJOINT(KERNEL) KERNEL<<<grid, 128, 0, s>>>(*sc, fr, af, depth, hit, dl_ddepth, dl_dshade, partials)
   if (engine == MBR_ENGINE_PLAIN_FP64) {
-    if (bulb) ADJOINT((adjoint_kernel<double, true>));
-    else if (per_pixel) ADJOINT(adjoint_pixel_kernel<double>);
+    if (bulb && per_pixel) ADJOINT((adjoint_pixel_kernel<double, true>));
+    else if (bulb) ADJOINT((adjoint_kernel<double, true>));
+    else if (per_pixel) ADJOINT((adjoint_pixel_kernel<double, false>));
     else ADJOINT((adjoint_kernel<double, false>));
   } else {
-    if (bulb) ADJOINT((adjoint_kernel<float, true>));
-    else if (per_pixel) ADJOINT(adjoint_pixel_kernel<float>);
+    if (bulb && per_pixel) ADJOINT((adjoint_pixel_kernel<float, true>));
+    else if (bulb) ADJOINT((adjoint_kernel<float, true>));
+    else if (per_pixel) ADJOINT((adjoint_pixel_kernel<float, false>));
     else ADJOINT((adjoint_kernel<float, false>));
   }
 #undef ADJOINT
