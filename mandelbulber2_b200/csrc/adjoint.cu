@@ -598,7 +598,7 @@ extern "C" mbr_status mbr_adjoint(mbr_ctx *ctx, const mbr_camera *camera, const 
   // us; the Mandelbulb 64x60 60 / 14 us, 256x256 182 / 81 us, 512x505 1664 / 802
   // us); and without a shade gradient, where a hit has one estimate and seven
   // lanes of the group would idle (the whole call, per pixel / eight lanes:
-  // Mandelbulb 64x64 51 / 50 us, 160x160 53 / 75 us, 256x256 65 / 109 us, 400x400
+  // Mandelbulb 64x64 51 / 53 us, 160x160 53 / 75 us, 256x256 65 / 109 us, 400x400
   // 89 / 202 us; Mandelbox 100x100 53 / 67 us).
   const bool bulb = sc->slot[0].formula == MBR_FORMULA_MANDELBULB;
   const bool per_pixel = !dl_dshade || (!bulb && n >= 16384);
