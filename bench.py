@@ -107,32 +107,6 @@ DEFAULT_ENGINE = {"mandelbox_1080p_A": "wavefront_fp32", "mandelbox_1080p_B": "w
                   "batch_2048": "wavefront_auto"}
 
 
-def kernels_per_frame(engine: str, p, formula: str, pixels: int) -> int:
-    """Kernel launches of one frame: the plain engines launch one kernel, or
-    stages P, N, S (shadow or AO) and the finish kernel for FP64 frames with 4
-    AO rays or 2^18 pixels and more (never the Menger sponge or GI); the
-    wavefront pipeline launches stage P, N (normals wanted), D and S (shadow or
-    AO), the finish kernel and the pixel counter; a GI frame launches the
-    primary paths, per bounce level (bounces + 1 of them) the normal and vertex
-    stages, the per-pixel sum and the pixel counter; the auto engine launches
-    the policy kernel and both pipelines, whose kernels of the precision not
-    chosen return at once."""
-    marches = p.ao_rays > 0 or (p.shading_enable and p.shadow_enable)
-    if "wavefront" not in engine:
-        staged = ("fp64" in engine and p.gi_samples == 0 and formula != "menger"
-                  and (p.ao_rays >= 4 or pixels >= 1 << 18))
-        return (4 if marches else 3) if staged else 1
-    if p.gi_samples > 0:
-        n = 1 + 2 * (p.gi_bounces + 1) + 2
-        return 1 + 2 * n if engine == "wavefront_auto" else n
-    n = 4  # primary, normals (the bench asks for normals), finish, pixel count
-    if marches:
-        n += 2  # directions, shadow/AO marches
-    if engine == "wavefront_auto":
-        return 1 + 2 * n
-    return n
-
-
 # ---- clocks ---------------------------------------------------------------------
 class ClockSampler:
     """SM clock and clock-event reasons sampled every 2 ms during the timed
@@ -249,7 +223,8 @@ def l2_flush_buffer(torch, device):
 
 
 def time_engine(r, torch, cam, p, bufs, engine, steps, warmup, flush, dist, world):
-    """Renders warmup + steps frames; returns (device seconds max over ranks, stats of the timed steps, per-step ms)."""
+    """Renders warmup + steps frames; returns (device seconds max over ranks, stats of the timed steps, per-step ms,
+    kernels of the library launched in the timed steps)."""
     from mandelbulber2_b200.render import STATS_FIELDS, stats_dict
 
     dev = r.device
@@ -263,11 +238,13 @@ def time_engine(r, torch, cam, p, bufs, engine, steps, warmup, flush, dist, worl
     if dist is not None:
         dist.barrier()
     torch.cuda.synchronize(dev)
+    launches = r.lib.mbr_kernel_launches()
     for k in range(steps):
         flush.fill_(float(k))  # L2 flush: a 256 MiB write between timed frames (outside the events)
         evs[k][0].record(stream)
         r.render_into(cam, p, bufs, stats, engine)
         evs[k][1].record(stream)
+    launches = r.lib.mbr_kernel_launches() - launches
     torch.cuda.synchronize(dev)
     r.sync()
     if dist is not None:
@@ -278,7 +255,7 @@ def time_engine(r, torch, cam, p, bufs, engine, steps, warmup, flush, dist, worl
         tt = torch.tensor([t], dtype=torch.float64, device=dev)
         dist.all_reduce(tt, op=dist.ReduceOp.MAX)
         t = float(tt.item())
-    return t, stats_dict(stats), ms
+    return t, stats_dict(stats), ms, launches
 
 
 def compare_frames(fast: dict, ref: dict) -> dict:
@@ -468,10 +445,12 @@ def run_batch(a, torch, dist, world, rank, local) -> None:
     if dist is not None:
         dist.barrier()
     torch.cuda.synchronize()
+    launches = lib.mbr_kernel_launches()
     e0.record()
     for _ in range(a.steps):
         lib.mbr_batch_launch(b, C.c_void_p(s.cuda_stream))
     e1.record()
+    launches = lib.mbr_kernel_launches() - launches
     torch.cuda.synchronize()
     clk = clocks.stop()
     r.sync()
@@ -536,7 +515,7 @@ def run_batch(a, torch, dist, world, rank, local) -> None:
                 "mpix_per_s": sd["pixels"] / t / 1e6, "stats_per_step": {k: v / a.steps for k, v in sd.items()},
                 "fp64_baseline": base, "speedup_vs_fp64": value / base["value"] if base else None,
                 "wall_speedup_vs_fp64": (base["seconds"] / (t / a.steps)) if base else None,
-                "gpu_launches": a.steps * n_groups * 4, "clocks": clk}
+                "gpu_launches": launches, "clocks": clk}
         print(json.dumps(line), flush=True)
     r.close()
 
@@ -600,7 +579,7 @@ def main() -> None:
 
     clocks = ClockSampler(local, pci_bus_id(torch, local))
     clocks.start()
-    t, st, ms = time_engine(r, torch, cam, p, bufs, engine, a.steps, a.warmup, flush, dist, world)
+    t, st, ms, launches = time_engine(r, torch, cam, p, bufs, engine, a.steps, a.warmup, flush, dist, world)
     clk = clocks.stop()
     de_total = torch.tensor([st["de_evals"], st["pixels"], st["formula_iterations"]], dtype=torch.float64,
                             device=r.device)
@@ -616,7 +595,7 @@ def main() -> None:
     if not a.no_baseline:
         bbufs = alloc_outputs(n, r.device, names)
         bsteps = max(1, min(a.steps, 3))
-        bt, bst, bms = time_engine(r, torch, cam, p, bbufs, base_engine, bsteps, 1, flush, dist, world)
+        bt, bst, bms, _ = time_engine(r, torch, cam, p, bbufs, base_engine, bsteps, 1, flush, dist, world)
         btot = torch.tensor([bst["de_evals"]], dtype=torch.float64, device=r.device)
         if dist is not None:
             dist.all_reduce(btot)
@@ -707,7 +686,7 @@ def main() -> None:
             "de_evals_per_frame": st["de_evals"] / a.steps, "stats_per_frame": {k: v / a.steps for k, v in st.items()},
             "fp64_baseline": base, "speedup_vs_fp64": (value / base["value"]) if base else None,
             "error_vs_fp64": err, "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
-            "gpu_launches": a.steps * kernels_per_frame(a.engine, p, desc["formula"], cam.width * cam.height),
+            "gpu_launches": launches,
             "clocks": clk, "per_step_ms": ms,
         }
         print(json.dumps(line), flush=True)

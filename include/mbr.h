@@ -727,6 +727,12 @@ mbr_status mbr_fract_parse(const char *text, mbr_scene *scene, mbr_camera *camer
                            char *report, int32_t report_size);
 
 /* ---- measurement ------------------------------------------------------------ */
+/* Kernels of this library that the calling thread's calls have queued so far
+ * (mbr_fma_peak's left out).  A frame recorded into a graph counts when it is
+ * recorded, a batch's graph with each mbr_batch_launch.  No counterpart in the
+ * reference. */
+int64_t mbr_kernel_launches(void);
+
 /* FMA throughput of the current device (FLOP/s, an FMA counted as 2), FP32
  * (fp64 = 0) or FP64: the roofline denominator for the DE kernels, which are
  * bound by the FMA/SFU pipes.  Synchronous.  No counterpart in the reference. */

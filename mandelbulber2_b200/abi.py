@@ -238,6 +238,7 @@ PROTOTYPES = {
     "mbr_batch_launch": (C.c_int, [_P, _P]),
     "mbr_batch_destroy": (None, [_P]),
     "mbr_batch_groups": (C.c_int32, [_P, _P]),
+    "mbr_kernel_launches": (C.c_int64, []),
     "mbr_wavefront_scratch_layout": (C.c_int, [C.c_int64, C.c_int32, C.POINTER(C.c_uint64),
                                                C.POINTER(C.c_uint64)]),
     "mbr_choose_precision": (C.c_int, [_P, _P, _P, _P]),

@@ -621,5 +621,6 @@ extern "C" mbr_status mbr_adjoint(mbr_ctx *ctx, const mbr_camera *camera, const 
   }
 #undef ADJOINT
   adjoint_sum_kernel<<<1, 32 * MBR_GRAD_COUNT, 0, s>>>(partials, grid, grad);
+  count_launches(2);
   return cuda_err(ctx, int(cudaGetLastError()), "adjoint kernel launch");
 }

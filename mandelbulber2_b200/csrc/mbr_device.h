@@ -311,6 +311,10 @@ struct Counters {
 };
 
 // ---- launchers (one per translation unit) ---------------------------------
+// Adds to the number of kernels that the calling thread has queued
+// (mbr_kernel_launches): called beside every launch.
+void count_launches(int n);
+
 // Plain per-pixel kernels: rows [0, height) of the frame.
 int launch_plain_fp64(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *stream);
 int launch_plain_fp64_strict(const DevScene &sc, const DevFrame &fr, const DevOutputs &out, void *stream);

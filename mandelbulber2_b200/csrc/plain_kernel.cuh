@@ -311,6 +311,7 @@ int launch_plain_t(const DevScene &sc, const DevFrame &fr, const DevOutputs &out
       default: plain_kernel<T, R, 0, false, V><<<grid, block, 0, s>>>(sc, fr, out); break;
     }
   }
+  count_launches(1);
   return int(cudaGetLastError());
 }
 
@@ -361,6 +362,7 @@ int launch_distance_t(const DevScene &sc, const double *pts, int64_t n, double d
     }
 #undef REFILL
   }
+  count_launches(1);
   return int(cudaGetLastError());
 }
 

@@ -616,6 +616,7 @@ int ref_stages(const DevScene &sc, const DevFrame &fr, const RefLaunch &L, const
   ref_primary_kernel<PM, FK, V><<<grid, 128, 0, s>>>(sc, fr, L, out);
   if (L.need_normal) ref_normal_kernel<PN, FK, V><<<grid, 128, 0, s>>>(sc, fr, L, out);
   if (L.per > 0) ref_shade_kernel<PM, FK, EXT, V><<<grid_s, 128, 0, s>>>(sc, fr, L, out);
+  count_launches(1 + (L.need_normal ? 1 : 0) + (L.per > 0 ? 1 : 0));
   return int(cudaGetLastError());
 }
 
@@ -679,6 +680,7 @@ int launch_staged_plain_t(const DevScene &sc, const DevFrame &fr, const DevOutpu
 #undef PASS
   if (e) return e;
   ref_finish_kernel<V><<<sm_count() * 4, 256, 0, s>>>(fr, L, out);
+  count_launches(1);
   return int(cudaGetLastError());
 }
 

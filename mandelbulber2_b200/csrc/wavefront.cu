@@ -211,6 +211,7 @@ mbr_status render_wavefront(mbr_ctx *ctx, const DevScene &sc, const DevFrame &fr
     int *gate = gi ? reinterpret_cast<int *>(reinterpret_cast<char *>(work) + 4096) : scratch_gate(work);
     L.gate = gate;
     policy_kernel<<<1, 32, 0, s>>>(sc, fr, gate);
+    count_launches(1);
     e = int(cudaGetLastError());
   }
   if (!e && engine != MBR_ENGINE_WAVEFRONT_FP64)
@@ -245,6 +246,7 @@ struct mbr_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   long long total = 0;
+  int launches = 0;  // kernels in the graph
   std::vector<BatchGroup> groups;
 };
 
@@ -281,6 +283,7 @@ static int batch_policy(const std::vector<DevScene> &dsc, const std::vector<int>
   if (!e) e = int(cudaMemcpy(d_wj, wj.data(), sizeof(WJob) * n, cudaMemcpyHostToDevice));
   if (!e) {
     batch_policy_kernel<<<(n + 127) / 128, 128>>>(d_sc, d_of, d_wj, n, fr0, d_fl);
+    count_launches(1);
     e = int(cudaGetLastError());
   }
   flags->assign(n, 0);
@@ -431,6 +434,7 @@ mbr_status mbr_batch_create(mbr_ctx *ctx, const mbr_scene *scenes, int32_t n_sce
     e = int(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
   }
   if (!e) {
+    const int64_t before = mbr_kernel_launches();
     int le = side_by_side ? int(cudaEventRecord(events[0], cs)) : 0;
     char *scratch = static_cast<char *>(b->d_scratch);
     std::vector<size_t> order, forked;
@@ -476,6 +480,8 @@ mbr_status mbr_batch_create(mbr_ctx *ctx, const mbr_scene *scenes, int32_t n_sce
       if (!je) je = int(cudaStreamWaitEvent(cs, events[i + 1], 0));
       if (!le) le = je;
     }
+    b->launches = int(mbr_kernel_launches() - before);  // recorded, not queued
+    count_launches(-b->launches);
     cudaGraph_t gr = nullptr;
     e = int(cudaStreamEndCapture(cs, &gr));
     b->graph = gr;
@@ -495,6 +501,7 @@ mbr_status mbr_batch_create(mbr_ctx *ctx, const mbr_scene *scenes, int32_t n_sce
 mbr_status mbr_batch_launch(mbr_batch *b, void *stream) {
   if (!b) return MBR_EINVAL;
   const int e = int(cudaGraphLaunch(b->exec, static_cast<cudaStream_t>(stream)));
+  if (!e) count_launches(b->launches);
   return cuda_err(b->ctx, e, "cudaGraphLaunch");
 }
 
@@ -522,6 +529,7 @@ mbr_status mbr_choose_precision(mbr_ctx *ctx, const mbr_camera *camera, const mb
   int e = int(cudaMalloc(&d_flag, sizeof(int)));
   if (e) return cuda_err(ctx, e, "cudaMalloc(flag)");
   policy_kernel<<<1, 32>>>(*sc, fr, d_flag);
+  count_launches(1);
   e = int(cudaGetLastError());
   int flag = 0;
   if (!e) e = int(cudaMemcpy(&flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost));

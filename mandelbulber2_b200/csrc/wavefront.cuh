@@ -1959,6 +1959,7 @@ static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const 
     break;
         GI_CASES(GP_LAUNCH)
 #undef GP_LAUNCH
+        count_launches(1);
       }
       for (int b = 0; b <= fr.gi_bounces; b++) {
         Launch Lb = L;
@@ -1977,10 +1978,12 @@ static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const 
     break;
         GI_CASES(GV_LAUNCH)
 #undef GV_LAUNCH
+        count_launches(2);
       }
 #undef GI_CASES
       gi_finish_kernel<<<sms * 4, 256, 0, st>>>(fr, j0, L, out, pixels);
       pixel_count_kernel<<<1, 32, 0, st>>>(L, out, pixels);
+      count_launches(2);
       return int(cudaGetLastError());
     }
   }
@@ -2023,6 +2026,7 @@ static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const 
 #undef STAGE_LAUNCH
   finish_kernel<<<sms * 4, 256, 0, st>>>(fr, L, out);
   pixel_count_kernel<<<1, 32, 0, st>>>(L, out, pixels);
+  count_launches(3 + (need_normal ? 1 : 0) + (marches ? 2 : 0));
   return int(cudaGetLastError());
 }
 
