@@ -151,7 +151,7 @@ struct DevScene {
   int32_t uniform_formula; // formula id when every iteration uses slot 0, else 0
   int32_t has_w;           // initial w != 0 or a 4-D formula (4-D state needed)
   int32_t generic;         // a slot's formula has no specialised FP32/FP64 form (reference-order iteration only)
-  int32_t pad1;
+  uint32_t orbit_slots;    // bit k: slot k is in the sequence table
   double julia_c[3];
   double cmul[3];
   double w0;
@@ -209,13 +209,14 @@ __host__ __device__ inline bool scene_extended(const DevScene &sc) {
          sc.delta_de || sc.de_final > DEF_LINEAR_OFFSET || sc.n_nodes > 0;
 }
 
-// Calls f with every slot that a pass of the scene's orbit can run: the entries
-// of the sequence table (an orbit longer than the table repeats the first).  An
-// empty slot is among them where no slot is live at iteration 0: the table is
-// then one entry long and names slot 0, whatever it holds.
+// Calls f with every slot that a pass of the scene's orbit can run: those in
+// the sequence table (an orbit longer than the table repeats its first entry).
+// An empty slot is among them where no slot is live at iteration 0: the table
+// is then one entry long and names slot 0, whatever it holds.
 template <class Fn>
 inline void for_orbit_slots(const DevScene &sc, Fn f) {
-  for (int i = 0; i < sc.length; i++) f(sc.slot[sc.seq[i]]);
+  for (int k = 0; k < MBR_MAX_FRACTALS; k++)
+    if (sc.orbit_slots >> k & 1u) f(sc.slot[k]);
 }
 
 // Whether a pass blends: a slot of the orbit has a weight other than 1 (an

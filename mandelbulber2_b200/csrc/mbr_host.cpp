@@ -631,6 +631,7 @@ mbr_status build_scene(mbr_ctx *ctx, const mbr_scene &sc, DevScene *out) {
   }
   if (rapidEnd) length = last + 1;
   d.length = length;
+  for (int i = 0; i < length; i++) d.orbit_slots |= 1u << d.seq[i];
 
   // DE function (hybrid_fractal_sequences.cpp:377-485)
   if (hybrid) {
