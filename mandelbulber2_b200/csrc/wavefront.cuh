@@ -760,8 +760,10 @@ __device__ __forceinline__ void flush_counts(const DevOutputs &out, unsigned int
 // 0.94 to 1.06, 1280x720 1.00 to 1.06 / 0.95 to 1.10 / 0.82 to 1.08, 640x360 0.99
 // to 1.02 / 0.94 to 1.03 / 0.89 to 1.03.  64 registers are best on the view that
 // fills the frame with short orbits and cost where orbits are long; 85 cost 1 %
-// at most.  Below, no bound: 320x180 0.98 to 0.99 / 0.91 to 0.95 / 0.89 to 0.94
-// (the Mandelbulb's is best unbounded, 512x512: 321 / 366 / 317 / 346 us).
+// at most.  From kManyPixels 64, which there cost on no view more than no bound
+// (the benchmark frame 5.94 ms, at 85 6.00); below kFewPixels no bound: 320x180
+// 0.98 to 0.99 / 0.91 to 0.95 / 0.89 to 0.94.  (The Mandelbulb's is best
+// unbounded, 512x512: 321 / 366 / 317 / 346 us.)
 template <int FK, bool MULTI, class P>
 struct kMinBlocks {
   static constexpr bool box64 = P::kWide && FK == FK_BOX_SIMPLE;
@@ -1915,8 +1917,9 @@ static int sm_count() {
   return sms;
 }
 
-// Below this many pixels the FP32 Mandelbox's stage P runs unbounded (see kMinBlocks).
-const long long kFewPixels = 131072;
+// The FP32 Mandelbox's stage P runs unbounded below the first number of pixels
+// and at 64 registers from the second (see kMinBlocks).
+const long long kFewPixels = 131072, kManyPixels = 1572864;
 
 // The stage launches of one frame or batch under policy P, in stream order.
 template <bool MULTI, class P>
@@ -2001,12 +2004,15 @@ static int launch_pipeline(int fk, const mbr_tuning &tu, cudaStream_t st, const 
     STAGE_LAUNCH(PP, KERNEL, FK_ANY, __VA_ARGS__)                                       \
     default: return int(cudaErrorInvalidValue);                                         \
   }
-  bool few = false;
+  bool primary = false;
   if constexpr (kMinBlocks<FK_BOX_SIMPLE, MULTI, P>::box32) {
-    few = fk == FK_BOX_SIMPLE && L.total < kFewPixels;
-    if (few) primary_kernel<FK_BOX_SIMPLE, MULTI, P, 0><<<grid, block, 0, st>>>(fr, fp0, j0, L, out);
+    primary = fk == FK_BOX_SIMPLE && (L.total < kFewPixels || L.total >= kManyPixels);
+    if (primary && L.total < kFewPixels)
+      primary_kernel<FK_BOX_SIMPLE, MULTI, P, 0><<<grid, block, 0, st>>>(fr, fp0, j0, L, out);
+    else if (primary)
+      primary_kernel<FK_BOX_SIMPLE, MULTI, P, 4><<<grid, block, 0, st>>>(fr, fp0, j0, L, out);
   }
-  if (!few) { STAGE(primary_kernel, fr, fp0, j0, L, out) }
+  if (!primary) { STAGE(primary_kernel, fr, fp0, j0, L, out) }
   const bool need_normal = fr.shading_enable || L.ao_rays > 0 || L.want_normal;
   if (need_normal) { typedef typename P::Normal PN; STAGEP(PN, normal_kernel, fr, fp0, L, out) }
   const bool marches = L.ao_rays > 0 || L.shadow_tasks > 0;

@@ -28,18 +28,20 @@ def test_bands_equal_the_frame(renderer, formula, engine):
         assert torch.equal(bufs[k], whole[k]), k
 
 
-@pytest.mark.parametrize("ao_rays", [0, 2])
-def test_fp32_mandelbox_bands(renderer, ao_rays):
-    """The FP32 Mandelbox's stage P has two register bounds by the number of pixels: the same bits from both."""
+@pytest.mark.parametrize("ao_rays,width,height,bands", [
+    (0, 512, 300, ((0, 140), (140, 300))), (2, 512, 300, ((0, 140), (140, 300))),
+    (1, 1536, 1024, ((0, 60), (60, 1000), (1000, 1024)))])
+def test_fp32_mandelbox_bands(renderer, ao_rays, width, height, bands):
+    """The FP32 Mandelbox's stage P has three register bounds by the number of pixels: the same bits from each."""
     import torch
 
     renderer.set_scene(configs.mandelbox_scene(2.2, 0.4, 40))
-    cam = configs.camera((3.0, -9.0, 3.0), width=512, height=300)
+    cam = configs.camera((3.0, -9.0, 3.0), width=width, height=height)
     p = configs.base_params(5, 30.0)
     p.ao_rays = ao_rays
     whole = renderer.render(cam, p, abi.ENGINE_WAVEFRONT_FP32, outputs=NAMES)
     bufs = alloc_outputs(cam.width * cam.height, renderer.device, NAMES)
-    for r0, r1 in ((0, 140), (140, 300)):
+    for r0, r1 in bands:
         renderer.render_into(cam, band_params(p, r0, r1), bufs, None, abi.ENGINE_WAVEFRONT_FP32)
     renderer.sync()
     for k in NAMES:
