@@ -566,6 +566,12 @@ __global__ void __launch_bounds__(256) ref_finish_kernel(const __grid_constant__
 //    1274 / 1513, 640x480 3077 / 2671, 1024x768 7490 / 5316; with 4 AO rays 64x48
 //    322 / 296, 400x300 2041 / 1871, 1024x768 14449 / 7001; Mandelbox without AO
 //    256x192 233 / 257, 640x480 1076 / 776.
+// The gain depends on the view.  Two Mandelboxes, the Mandelbulb and two
+// sequences from four sides, 4 rays: 128x96 0.81 to 1.75 (mean 1.28), 320x240 0.83
+// to 1.97 (1.29), 640x480 0.91 to 2.82 (1.76), 800x600 1.13 to 2.99; 8 rays 0.89 at
+// the least, 16 rays 1.04.  It is below 1 where one ray's chain of estimates sets
+// the time, which takes longer in stages than in a warp of its own: the Mandelbox
+// seen from above an edge up to 640x480, the Mandelbulb's limb at 128x96.
 // The size is the frame's, whatever rows of it are asked for: a band of a frame
 // has to equal the frame's rows bit for bit, so it takes the frame's kernels.
 inline bool staged_plain_takes(const DevScene &sc, const DevFrame &fr) {

@@ -158,7 +158,7 @@ mbr_status render_wavefront(mbr_ctx *ctx, const DevScene &sc, const DevFrame &fr
   if (!is_wavefront(engine)) return set_err(ctx, MBR_EINVAL, "not a wavefront engine: %d", engine);
   mbr_status stt = check_supported(ctx, sc, fr, false);
   if (stt != MBR_OK) return stt;
-  // hybrids and formulas without a specialised form iterate in the reference's order (PrecHyb)
+  // hybrids and formulas without a specialised form iterate in the reference's order (PrecHybT)
   const bool gi = fr.gi_samples > 0, hyb = sc.is_hybrid != 0 || sc.generic != 0;
   if (gi && fr.gi_bounces > 120)
     return set_err(ctx, MBR_EUNSUPPORTED, "wavefront engine: GI with more than 120 bounces uses the plain engines");

@@ -481,7 +481,8 @@ struct PrecHybT {
 
   // |z|^2 with its fused operations spelled out, so that every kernel and
   // every feature set rounds alike: x before y, at the starting point of a
-  // normal sample y before x.
+  // normal sample y before x, the order of the general kernels, whose len4 the
+  // compiler fuses (tests/test_gpu_hybrid_rounding.py compares their bits).
   __device__ static float square_of(const V4<float> &z) { return fmaf(z.z, z.z, fmaf(z.x, z.x, __fmul_rn(z.y, z.y))); }
   __device__ static float start_square_of(const V4<float> &z) {
     if (!(FEAT & HB_NORMAL)) return square_of(z);

@@ -4,9 +4,12 @@
 namespace mbr {
 
 // The kernels by what the scene needs: single formulas of the three with
-// extensions, sequences of the three, and a general kernel of each kind that
+// extensions; sequences of the Mandelbulb and the Menger sponge, of the Mandelbox
+// and the Menger sponge, and of all three; and a general kernel of each kind that
 // also takes blended slots and fast AO (the extended one: GI and every other
-// formula).  The general kernels alone against this choice: an 800x600
+// formula).  Sequences of the Mandelbulb and the Mandelbox alone take the
+// three-formula kernel: in one of the two the compiler fused other operations of
+// the Mandelbox, and its frames differed from the general kernel's in last bits.  The general kernels alone against this choice: an 800x600
 // Mandelbox with primitives 8.46 / 4.12 ms (its parameters become constant
 // operands and 16 formulas leave the loop), 1080p x 16 spp GI of a
 // Mandelbulb and Menger sequence 187.5 / 154.5 ms.
