@@ -181,7 +181,10 @@ __device__ __forceinline__ void f_mandelbox(V4<T> &z, T &DE, const DevSlot &s, c
   DE = DE * P<T>(s, P_MB_ABS_SCALE) + T(1.0);
 }
 
-template <class T, bool W>
+// SPLIT: the product z.z s3, which is compared and may have 2 taken off, stays
+// rounded by itself; left to the compiler, the two are fused or not by what
+// surrounds them.
+template <class T, bool W, bool SPLIT = false>
 __device__ __forceinline__ void f_menger(V4<T> &z, T &DE, const DevSlot &s) {
   z.x = m_abs(z.x);
   z.y = m_abs(z.y);
@@ -198,7 +201,10 @@ __device__ __forceinline__ void f_menger(V4<T> &z, T &DE, const DevSlot &s) {
   if (W) z.w = z.w * s3;
   z.x = z.x - T(2.0);
   z.y = z.y - T(2.0);
-  if (z.z > T(1.0)) z.z = z.z - T(2.0);
+  if (z.z > T(1.0)) {
+    if constexpr (SPLIT && sizeof(T) == 4) z.z = __fadd_rn(z.z, -2.0f);
+    else z.z = z.z - T(2.0);
+  }
   DE = DE * s3;
 }
 
@@ -1332,8 +1338,8 @@ __device__ __noinline__ void call_menger_mod1(V4<T> &z, T &DE, const DevSlot &s,
 // rotations are compiled in; kernels of scenes that use none of them (hybrids
 // of the three included) are built without that code.
 // i: the iteration (aux.i); c: the orbit's c (aux.const_c), which the Aexion
-// replaces at its first iteration.
-template <class T, bool W, bool EXT = false>
+// replaces at its first iteration.  SPLIT: see f_menger.
+template <class T, bool W, bool EXT = false, bool SPLIT = false>
 __device__ __forceinline__ void formula_dispatch(int formula, V4<T> &z, T r, T &DE, const DevSlot &s,
                                                  const MbRot *rot, const IfsBlock *ifs, int i, V4<T> &c,
                                                  AuxX<T> &ax) {
@@ -1357,7 +1363,7 @@ __device__ __forceinline__ void formula_dispatch(int formula, V4<T> &z, T r, T &
       case MBR_FORMULA_HYPERCOMPLEX: f_hypercomplex<T>(z, r, DE); break;
       case MBR_FORMULA_KALEIDOSCOPIC_IFS: f_ifs<T>(z, DE, *ifs); break;
       case MBR_FORMULA_XENODREAMBUIE: f_xenodreambuie<T>(z, r, DE, s); break;
-      default: f_menger<T, W>(z, DE, s); break;
+      default: f_menger<T, W, SPLIT>(z, DE, s); break;
     }
   } else {
     switch (formula) {

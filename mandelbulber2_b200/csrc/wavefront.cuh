@@ -489,6 +489,28 @@ struct PrecHybT {
     return fmaf(z.z, z.z, fmaf(z.y, z.y, __fmul_rn(z.x, z.x)));
   }
 
+  // smooth4 (SmoothCVector) in the sequences' kernel, its first length given:
+  // |z| as the pass before rounded it, except in every fourth pass, which
+  // computes it anew with the other fused operation first.  Which of the two it
+  // is shows in the last bits only, but also in iteration counts and 8-bit
+  // colours of single pixels; the orbits keep the rounding of a loop whose
+  // passes come in groups of four (tests/test_gpu_blended_bits.py).
+  __device__ static float last_length(int i, float r, const V4<float> &z) {
+    if (i & 3) return r;
+    if (FEAT & HB_NORMAL) return sqrtf(square_of(z));
+    return sqrtf(fmaf(z.z, z.z, fmaf(z.y, z.y, __fmul_rn(z.x, z.x))));
+  }
+  __device__ static V4<float> blend(const V4<float> &v1, const V4<float> &v2, double k, float l1) {
+    if (k <= 0.0) return v1;
+    const float kk = float(k), nk = float(1.0 - k);
+    const float l2 = len4<float, false>(v2);
+    const float length = l1 * nk + l2 * kk;
+    const V4<float> t{v1.x * nk + v2.x * kk, v1.y * nk + v2.y * kk, v1.z * nk + v2.z * kk, 0.0f};
+    const float lt = len4<float, false>(t);
+    if (lt > 0.0f) return V4<float>{t.x / lt * length, t.y / lt * length, t.z / lt * length, 0.0f};
+    return v1;
+  }
+
   template <int FK>
   __device__ static void start(State &e, const Params &, float qx, float qy, float qz) {
     e.zx = qx;
@@ -526,7 +548,7 @@ struct PrecHybT {
         // the Aexion, the one formula that replaces c, is 4-D and never runs here
         V4<float> c{e.cx, e.cy, e.cz, 0.0f};
         AuxX<float> ax{1.0f, 0.0f, 0.0f, 1.0f, 1000.0f, c};  // formulas with orbit state do not run here (check_supported)
-        formula_dispatch<float, false, true>(s.formula, z, r, de, s, &sc.mbrot, &sc.ifs, i, c, ax);
+        formula_dispatch<float, false, true, true>(s.formula, z, r, de, s, &sc.mbrot, &sc.ifs, i, c, ax);
       } else {
         constexpr int F = FEAT & (HB_BULB | HB_BOX | HB_MENGER);
         if ((FEAT & HB_BULB) && (F == HB_BULB || s.formula == MBR_FORMULA_MANDELBULB))
@@ -534,7 +556,7 @@ struct PrecHybT {
         else if ((FEAT & HB_BOX) && (!(FEAT & HB_MENGER) || s.formula == MBR_FORMULA_MANDELBOX))
           f_mandelbox<float, false, EXT>(z, de, s, &sc.mbrot);
         else
-          f_menger<float, false>(z, de, s);
+          f_menger<float, false, true>(z, de, s);
       }
     }
     if (s.add_c) {
@@ -551,7 +573,7 @@ struct PrecHybT {
     if ((FEAT & HB_BLEND) && sc.is_hybrid) {
       const double kw = s.d[P_WEIGHT];
       if (kw < 1.0) {
-        z = smooth4<float, false>(tempZ, z, kw);
+        z = EXT ? smooth4<float, false>(tempZ, z, kw) : blend(tempZ, z, kw, last_length(i, e.r, tempZ));
         de = de * float(kw) + tempDE * float(1.0 - kw);
       }
     }
