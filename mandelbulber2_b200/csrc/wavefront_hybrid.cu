@@ -27,7 +27,9 @@ int pipeline_hybrid(const DevScene &sc, const mbr_tuning &tu, cudaStream_t st, c
                                              : HB_ALL;
   });
   if (scene_extended(sc)) {
-    if (!sc.is_hybrid && !blend && fr.gi_samples == 0 && !L.ao_fast) {
+    // (the pseudo-Kleinian DE function's x^2 + y^2 shares products with the lean
+    // kernels' |z|^2, and the compiler fuses it otherwise than in the general one)
+    if (!sc.is_hybrid && !blend && fr.gi_samples == 0 && !L.ao_fast && sc.de_final != DEF_PSEUDO_KLEINIAN) {
       if (forms == HB_BOX) HYBRID(HB_EXT | HB_BOX);
       if (forms == HB_BULB) HYBRID(HB_EXT | HB_BULB);
       if (forms == HB_MENGER) HYBRID(HB_EXT | HB_MENGER);

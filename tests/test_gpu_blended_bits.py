@@ -1,9 +1,9 @@
-"""Blended sequences, and sequences with extensions in GI, keep their bits on the
-FP32 wavefront: which products a compiler fuses in the blend and in the Menger
-sponge changes with the code around them, and with it the iteration counts and
-8-bit colours of single pixels.  The digests are of the frames of the kernels as
-they were before they were split by features; the orbits use no library
-function, only IEEE operations."""
+"""Blended sequences, sequences with extensions in GI, and the pseudo-Kleinian DE
+function keep their bits on the FP32 wavefront: which products a compiler fuses
+in the blend, in the Menger sponge and in that function changes with the code
+around them, and with it the iteration counts and 8-bit colours of single pixels.
+The digests are of the frames of the kernels as they were before they were split
+by features; the orbits use no library function, only IEEE operations."""
 import hashlib
 
 import pytest
@@ -15,6 +15,12 @@ NAMES = ("depth", "iters", "hit", "normal", "shade", "ao", "rgb", "rgb8")
 
 
 def _scene(name):
+    if name.endswith("kleinian_de"):
+        sc = configs.menger_scene(5) if name.startswith("menger") else configs.mandelbox_scene(-1.5, 0.5, 9)
+        sc.delta_de_function = 3  # pseudo-Kleinian
+        sc.julia_mode = 1
+        sc.julia_c[:] = [0.3, -0.2, 0.1]
+        return sc
     sc = configs.mandelbox_scene(-1.5, 0.5, 30)
     sc.hybrid_fractal_enable = 1
     sc.n_fractals = 2
@@ -35,7 +41,7 @@ def _scene(name):
 
 def digest(renderer, name, kind):
     renderer.set_scene(_scene(name))
-    cam = configs.camera((1.8, -5.4, 2.1), width=160, height=120)
+    cam = configs.camera((1.8, -5.4, 2.1) if name != "menger_kleinian_de" else (0.7, -2.2, 0.9), width=160, height=120)
     if kind == "gi":
         _, _, p = configs.hybrid_gi_2160p(160, 120, spp=2)
         p.gi_bounces = 3
@@ -53,6 +59,8 @@ def digest(renderer, name, kind):
 
 
 DIGESTS = {
+    ("menger_kleinian_de", "ao"): "c03874d6aba3fc7f", ("menger_kleinian_de", "gi"): "e758b48b7fb839d3",
+    ("box_kleinian_de", "ao"): "1f6558da8f0581fc",
     ("box", "ao"): "63a0a821407b782a", ("box", "fast"): "a3cf4ad85658f99d", ("box", "gi"): "185b5e58a052f26e",
     ("menger", "ao"): "f6194b13ac09d97f", ("menger", "fast"): "a12cc7497dbf2964", ("menger", "gi"): "f8ff231aef030372",
     ("limits", "ao"): "ab2c26183b5e105d", ("limits", "fast"): "923ed0e032d584f1", ("limits", "gi"): "d541ee2a0a3a6801",
